@@ -11,6 +11,7 @@ void cheb_table_sizes(const Dims &d, size_t *nsyn, size_t *nana);
 // cana may be null (synthesis matrix only)
 void launch_cheb_tables(const Dims &d, const double *cosy, double *csyn, double *cana, cudaStream_t s);
 cudaError_t configure_cheb_kernels(const Dims &d);
+cudaError_t configure_ysynth_kernel(const Dims &d);   // the FP64 synthesis alone
 // vorticity om[3][Ns] of u[3][Ns] and its pressure-wall sums bw[2][ncol] (bw may be null)
 void launch_curl(const Dims &d, const Tables &t, const double2 *u, double2 *om, double2 *bw, double re,
                  cudaStream_t s);

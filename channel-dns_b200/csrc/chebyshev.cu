@@ -526,8 +526,10 @@ void launch_cheb_tables_adjoint(const Dims &d, const double *cosy, double *csyn_
                                                  1.0 / ((double)d.NX2 * (double)d.NZ2));
 }
 
+cudaError_t configure_ysynth_kernel(const Dims &d) { return raise_smem(k_ysynth<double2>, syn_smem(d)); }
+
 cudaError_t configure_cheb_kernels(const Dims &d) {
-    cudaError_t e = raise_smem(k_ysynth<double2>, (int)syn_smem(d));
+    cudaError_t e = configure_ysynth_kernel(d);
     if (e == cudaSuccess)
         e = raise_smem(k_ysynth<float2>, (int)syn_smem(d));
     if (e == cudaSuccess)

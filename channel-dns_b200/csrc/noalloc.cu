@@ -164,6 +164,7 @@ extern "C" int cdns_transform_fine_backward_noalloc(const cdns_mesh_desc *m, con
         if (fresh) {
             g_table_mesh[dev].valid = false;
             e = configure_transform_kernels(d);
+            if (e == cudaSuccess) e = configure_ysynth_kernel(d);
             if (e != cudaSuccess) return record_error(CDNS_ERR_CUDA, cudaGetErrorString(e));
             g_table_mesh[dev].mesh = *m;
             g_table_mesh[dev].valid = true;

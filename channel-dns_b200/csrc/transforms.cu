@@ -17,6 +17,7 @@
 #include "cdns_kernels.cuh"
 #include "fft_lines.cuh"
 #include "reg_fft.cuh"
+#include "transform_ops.cuh"
 
 namespace cdns {
 
@@ -26,65 +27,6 @@ namespace cdns {
 // HBM into the NZ2 slots (negative Nyquist slot wins at a full z spectrum,
 // src/fft/transforms.cpp:715-732); the last pass writes z-physical rows.
 // ---------------------------------------------------------------------------
-// The coarse-grid transform (coarse = true, src/fft/transforms.cpp:560-572)
-// instead sums the two Nyquist coefficients into the shared slot.
-template <class C> struct ZExpandSrc {
-    const C *Fp;   // one (field, y point) plane [kz][kx]
-    int nkx, kx0, NZS, n;
-    bool coarse;
-    __device__ __forceinline__ C operator()(int z, int line) const {
-        const int kx = kx0 + line;
-        if (kx >= nkx) return mkc<C>(0, 0);
-        int kz;
-        if (z <= NZS) {
-            if (z == n - NZS) {
-                if (coarse) return cadd(Fp[(2 * NZS) * nkx + kx], Fp[kx]);
-                kz = -NZS;
-            } else {
-                kz = z;
-            }
-        } else if (z >= n - NZS) {
-            kz = z - n;
-        } else {
-            return mkc<C>(0, 0);
-        }
-        return Fp[(kz + NZS) * nkx + kx];
-    }
-};
-template <class C> struct RowDst {
-    C *p;   // [pos][kx]
-    int nkx, kx0;
-    __device__ __forceinline__ void operator()(int pos, int line, C v) const {
-        const int kx = kx0 + line;
-        if (kx < nkx) p[(long long)pos * nkx + kx] = v;
-    }
-};
-template <class C> struct RowSrc {
-    const C *p;
-    int nkx, kx0;
-    __device__ __forceinline__ C operator()(int pos, int line) const {
-        const int kx = kx0 + line;
-        return kx < nkx ? p[(long long)pos * nkx + kx] : mkc<C>(0, 0);
-    }
-};
-// Forward z: keep kz in [-NZS, NZS] scaled by 1/NZ2 (src/fft/transforms.cpp:658-665);
-// at a full z spectrum slot NZS feeds both kz = +NZS and kz = -NZS, halved on
-// the coarse grid (coarse = true, src/fft/transforms.cpp:506-511).
-template <class C> struct ZTruncDst {
-    C *Fp;
-    int nkx, kx0, NZS, n;
-    typename CReal<C>::T invn;
-    bool coarse;
-    __device__ __forceinline__ void operator()(int z, int line, C v) const {
-        const int kx = kx0 + line;
-        if (kx >= nkx) return;
-        C s = cscale(invn, v);
-        if (coarse && z <= NZS && z >= n - NZS) s = cscale((typename CReal<C>::T)0.5, s);
-        if (z <= NZS) Fp[(z + NZS) * nkx + kx] = s;
-        if (z >= n - NZS) Fp[(z - n + NZS) * nkx + kx] = s;
-    }
-};
-
 __global__ void __launch_bounds__(256, 2)
 k_z_backward(Dims d, FftPlan P, const double2 *__restrict__ roots, const double2 *__restrict__ F,
              double2 *__restrict__ G, int TL, bool coarse) {
@@ -121,18 +63,6 @@ k_z_forward(Dims d, FftPlan P, const double2 *__restrict__ roots, const double2 
 // Register form of the z transforms for NZ2 = N1 x N2: threads t = n2 TL + l
 // (step 1) and t = k1 TL + l (step 2) over TL kx lines, one shared-memory
 // exchange S[k1][n2][l]; loads and stores run along kx.
-// Shared twiddle table of the register forms: n double2 slots, holding the
-// FP64 roots, or the FP32 roots and their rounding residues.
-template <class C> __device__ __forceinline__ Twiddles<C> load_twiddles(double2 *sm_d, const double2 *roots, int n) {
-    C *hi = reinterpret_cast<C *>(sm_d);
-    C *lo = sizeof(C) == 8 ? hi + n : hi;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double2 r = roots[i];
-        hi[i] = cto<C>(r);
-        if (sizeof(C) == 8) lo[i] = mkc<C>(r.x - (double)hi[i].x, r.y - (double)hi[i].y);
-    }
-    return Twiddles<C>{hi, lo};
-}
 // Inter-step twiddles of an N1 x N2 register transform (N2 <= 16) as N1 rows of
 // 16: entry (k1, s) = exp(-2 pi i s k1 / n), in 16 N1 double2 slots (FP32: the
 // roots and their rounding residues).  The view returned is offset to the
@@ -148,11 +78,6 @@ __device__ __forceinline__ Twiddles<C> load_lane_twiddles(double2 *sm_d, const d
     }
     return Twiddles<C>{hi + sub, lo + sub};
 }
-
-// Row stride of fft2_lines' exchange between k1 groups: N2 TL padded to = TL
-// (mod 8), so that a quarter-warp whose threads span two k1 groups touches 8
-// distinct 16-byte bank groups (unpadded, N2 TL = 0 mod 8 for the even N2 used).
-__host__ __device__ constexpr int fft2_kstride(int n2, int tl) { return n2 * tl + (((tl - n2 * tl) % 8) + 8) % 8; }
 
 template <int N1, int N2, int SIGN, class C, class Src, class Dst>
 __device__ __forceinline__ void fft2_lines(int TL, const Twiddles<C> &tw, C *S, const Src &src, const Dst &dst) {
@@ -289,77 +214,46 @@ k_z_forward_peers(Dims d, const double2 *__restrict__ roots, const double2 *__re
 //             (the scalings 1/(2 NY2) and 1/NY2 with the DCT-I's doubled
 //             interior sum), k <= NYS.
 // Block = one (field, kz) plane x TL kx lines (TL a compile-time width), 16 TL
-// threads: thread t owns line l = t mod TL and row group r = t / TL (rows
-// r, r + 16, ...), so that in every phase consecutive threads touch
-// consecutive lines -- coalesced global rows along kx and conflict-free
-// shared rows [n][l].  Phases (barriers between):
-//   load x_n (n = 0..N) and each thread's partial of Y_1's sum over its rows;
-//   Z = DFT_N(y) (fft2_lines; the exchange aliases x, read before its barrier);
+// threads: thread t owns line l = t mod TL and row group r = t / TL, so that in
+// every phase consecutive threads touch consecutive lines -- coalesced global
+// rows along kx and conflict-free shared rows.  One shared array holds the
+// transform from load to output: row n of y at [n / N2][n mod N2] (row stride
+// TL, group stride fft2_kstride), which is where step 1's thread n2 = r reads
+// n2 + N2 n1 and leaves its frequencies k1, and where step 2's thread k1 = r
+// reads them and leaves Z_{k1 + N1 k2}: every thread writes only what it read,
+// so the steps need no second buffer and no barrier between read and write.
+// Phases (barriers between):
+//   load the pairs x_n, x_{N-n} (n = r, r + 16, ... <= N/2), write y_n and
+//   y_{N-n}, partial of Y_1's sum;
+//   step 1; step 2;
 //   even outputs from Z pairs, stored from registers, and each thread's chunk
 //   of the odd outputs' prefix sum (16 consecutive-k chunks per line);
 //   the carry of the earlier chunks (a fixed-order sum of their totals) and
 //   the odd outputs, stored from registers.  Stores run along kx (11-16 lines of
 //   one row per thread group), as the loads do.
-// Shared memory: twiddles [N], x / exchange [(N+1)][TL] (or the padded
-// exchange), Z [N][TL], partials [16][TL] (Y_1's, then the chunk totals), Y_1 [TL].
+// Bound by latency and the shared-memory pipe: at N = 192 the one array leaves 5
+// blocks of 176 threads per SM (41 KB each) where a separate x and Z took 3 of
+// 74 KB, and pairing drops one of seven shared passes.
+// Shared memory: twiddles [N], the array, partials [16][TL] (Y_1's, then the
+// chunk totals), Y_1 [TL].
 // ---------------------------------------------------------------------------
-struct YdctSrc {
-    const double2 *X;
-    const double *cosy;
-    int TL, N;
-    __device__ __forceinline__ double2 operator()(int n, int l) const {
-        const double2 a = X[n * TL + l], b = X[(N - n) * TL + l];
-        const double s = cosy[(n + (3 * N) / 2) % (2 * N)];   // sin(pi n / N)
-        return csub(cscale(0.5, cadd(a, b)), cscale(s, csub(a, b)));
-    }
-};
-struct YdctDst {
-    double2 *Z;
-    int TL;
-    __device__ __forceinline__ void operator()(int k, int l, double2 v) const { Z[k * TL + l] = v; }
-};
-
 constexpr int kYdctRows = 16;   // row groups of the DCT kernel (16 TL threads)
-// x / exchange region of the DCT kernel: the N + 1 rows, or the padded exchange
-__host__ __device__ constexpr int ydct_xslots(int n1, int n2, int tl) {
-    return (n1 * n2 + 1) * tl > n1 * fft2_kstride(n2, tl) ? (n1 * n2 + 1) * tl : n1 * fft2_kstride(n2, tl);
-}
 __host__ __device__ constexpr size_t ydct_slots(int n1, int n2, int tl) {
-    return (size_t)n1 * n2 + (size_t)ydct_xslots(n1, n2, tl) + (size_t)n1 * n2 * tl + (size_t)kYdctRows * tl + tl;
+    return (size_t)n1 * n2 + (size_t)n1 * fft2_kstride(n2, tl) + (size_t)kYdctRows * tl + tl;
 }
-
-// Operands of the DCT kernels; CT is the stage buffer's complex type (double2,
-// or float2 for the mixed form's FP32 stages).  Synthesis: spectral
-// spec0 / spec1 (fields f < nsplit / the rest), coefficient k weighted by
-// in0 (k = 0) or in1, -> F, row j weighted by outE (j = 0, N) or outI; with
-// `mean` (FP32 stages) the (kz, kx) = (0, 0) column goes to mean[f][j] in FP64
-// and zeros to F.  Analysis: F, row j weighted by inE (j = 0, N) or inI, ->
-// spectral S, coefficient k scaled by s0 (k = 0) or sk.  The forward
-// transforms take unit weights and s0 = 1/N, sk = 2/N (times 1 / (NX2 NZ2) for
-// FP32 stages, whose z and x analyses leave it out); the discrete adjoint's
-// transposed stages take other weights (launch_ydct_adjoint_*).
-template <class CT> struct YdctArgs {
-    const double2 *spec0 = nullptr, *spec1 = nullptr;
-    int nsplit = 0;
-    const CT *Fin = nullptr;
-    CT *Fout = nullptr;
-    double2 *S = nullptr;
-    double *mean = nullptr;
-    double in0 = 1.0, in1 = 1.0, outE = 1.0, outI = 1.0;   // synthesis weights
-    double inE = 1.0, inI = 1.0, s0 = 0.0, sk = 0.0;       // analysis weights and scales
-};
 
 template <int N1, int N2, bool ANA, int TL, class CT>
 __global__ void __launch_bounds__(16 * TL)
 k_ydct_r(Dims d, const double2 *__restrict__ roots, const double *__restrict__ cosy, YdctArgs<CT> A) {
     constexpr int N = N1 * N2;
     constexpr int R = kYdctRows;
+    constexpr int KS = fft2_kstride(N2, TL);
     constexpr int M = N / 2 - 1;                // odd outputs beyond Y_1: k = 1..M
     constexpr int CH = (N / 2 + R) / R;         // k = 0..N/2 in R chunks of CH
+    static_assert(N1 <= R && N2 <= R, "a row group per FFT thread");
     extern __shared__ double2 sm_d[];
-    double2 *X = sm_d + N;
-    double2 *Z = X + ydct_xslots(N1, N2, TL);
-    double2 *P = Z + N * TL;
+    double2 *Y = sm_d + N;
+    double2 *P = Y + N1 * KS;
     double2 *Y1 = P + R * TL;
     const int f = blockIdx.z, kzi = blockIdx.y, kx0 = blockIdx.x * TL;
     const int t = threadIdx.x;
@@ -367,55 +261,75 @@ k_ydct_r(Dims d, const double2 *__restrict__ roots, const double *__restrict__ c
     const int nkx = d.nkx, ncy = d.ncy, kx = kx0 + l;
     const bool lok = kx < nkx;
     const Twiddles<double2> tw = load_twiddles<double2>(sm_d, roots, N);
-    // ---- x_n, n = 0..N, and partials of Y_1 = sum_{n=1}^{N-1} x_n cos(pi n / N)
-    // rows n = r + R i: all loads of a thread are issued before the first use
-    constexpr int NI = N / R + 1;
-    double2 y1 = mk(0.0, 0.0);
-    double2 xv[NI];
+    auto row = [&](int n) { return (n / N2) * KS + (n % N2) * TL + l; };
+    // ---- y_n, y_{N-n} from x_n, x_{N-n}; partials of Y_1 = (x_0 - x_N)/2 +
+    // sum_{n=1}^{N-1} x_n cos(pi n / N); all loads are issued before the first use
+    constexpr int NI = N / 2 / R + 1;
+    double2 xa[NI], xb[NI];
     if (!ANA) {
         const double2 *S = (f < A.nsplit ? A.spec0 + (long long)f * d.Ns : A.spec1 + (long long)(f - A.nsplit) * d.Ns) +
                            (long long)kzi * ncy * nkx + kx;
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
-            const int n = r + R * i;
-            xv[i] = (n <= N && n < ncy && lok) ? S[(long long)n * nkx] : mk(0.0, 0.0);
-        }
-#pragma unroll
-        for (int i = 0; i < NI; ++i) {
-            const int n = r + R * i;
-            if (n > N) break;
-            double2 v = cscale(n == 0 ? A.in0 : A.in1, xv[i]);
-            if (n == 0) v = cadd(v, v);
-            X[n * TL + l] = v;
-            if (n >= 1 && n < N) y1 = cadd(y1, cscale(cosy[n], v));
+            const int n = r + R * i, m = N - n;
+            xa[i] = (n <= N / 2 && n < ncy && lok) ? S[(long long)n * nkx] : mk(0.0, 0.0);
+            xb[i] = (n <= N / 2 && m < ncy && lok) ? S[(long long)m * nkx] : mk(0.0, 0.0);
         }
     } else {
         const CT *F = A.Fin + (long long)f * d.ny2 * d.fcol + (long long)kzi * nkx + kx;
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
-            const int n = r + R * i;
-            xv[i] = (n <= N && lok) ? cto<double2>(F[(long long)n * d.fcol]) : mk(0.0, 0.0);
+            const int n = r + R * i, m = N - n;
+            xa[i] = (n <= N / 2 && lok) ? cto<double2>(F[(long long)n * d.fcol]) : mk(0.0, 0.0);
+            xb[i] = (n <= N / 2 && lok) ? cto<double2>(F[(long long)m * d.fcol]) : mk(0.0, 0.0);
         }
+    }
+    double2 y1 = mk(0.0, 0.0);
 #pragma unroll
-        for (int i = 0; i < NI; ++i) {
-            const int n = r + R * i;
-            if (n > N) break;
-            const double2 v = cscale(n == 0 || n == N ? A.inE : A.inI, xv[i]);
-            X[n * TL + l] = v;
-            if (n >= 1 && n < N) y1 = cadd(y1, cscale(cosy[n], v));
-        }
+    for (int i = 0; i < NI; ++i) {
+        const int n = r + R * i;
+        if (n > N / 2) break;
+        // x_0 of the synthesis is 2 c_0
+        const double w0 = !ANA ? (n == 0 ? 2.0 * A.in0 : A.in1) : (n == 0 ? A.inE : A.inI);
+        const double w1 = !ANA ? A.in1 : (n == 0 ? A.inE : A.inI);
+        const double2 a = cscale(w0, xa[i]), b = cscale(w1, xb[i]);
+        const double2 h = cscale(0.5, cadd(a, b)), df = csub(a, b);
+        const double sn = cosy[n < N / 2 ? n + (3 * N) / 2 : 0];   // sin(pi n / N)
+        y1 = cadd(y1, cscale(n == 0 ? 0.5 : cosy[n], df));   // cos(pi (N - n) / N) = -cos(pi n / N)
+        Y[row(n)] = csub(h, cscale(sn, df));
+        if (n > 0 && n < N / 2) Y[row(N - n)] = cadd(h, cscale(sn, df));
     }
     P[r * TL + l] = y1;
     __syncthreads();
     if (r == 0) {
-        double2 acc = cscale(0.5, csub(X[l], X[N * TL + l]));
+        double2 acc = P[l];
 #pragma unroll
-        for (int q = 0; q < R; ++q) acc = cadd(acc, P[q * TL + l]);
+        for (int q = 1; q < R; ++q) acc = cadd(acc, P[q * TL + l]);
         Y1[l] = acc;
     }
-    // ---- Z = DFT_N(y) (the exchange buffer aliases X: read before its barrier)
-    fft2_lines<N1, N2, -1>(TL, tw, X, YdctSrc{X, cosy, TL, N}, YdctDst{Z, TL});
+    // ---- Z = DFT_N(y), in place -------------------------------------------
+    if (r < N2) {
+        double2 v[N1];
+        double2 *q = Y + r * TL + l;
+#pragma unroll
+        for (int n1 = 0; n1 < N1; ++n1) v[n1] = q[n1 * KS];
+        dft_reg<N1, -1>(v, tw, N2);
+#pragma unroll
+        for (int k1 = 0; k1 < N1; ++k1)
+            q[k1 * KS] = (k1 == 0 || r == 0) ? v[k1] : tw.template mul<-1>(v[k1], r * k1);
+    }
     __syncthreads();
+    if (r < N1) {
+        double2 v[N2];
+        double2 *q = Y + r * KS + l;
+#pragma unroll
+        for (int m = 0; m < N2; ++m) v[m] = q[m * TL];
+        dft_reg<N2, -1>(v, tw, N1);
+#pragma unroll
+        for (int k2 = 0; k2 < N2; ++k2) q[k2 * TL] = v[k2];
+    }
+    __syncthreads();
+    auto Z = [&](int k) { return Y[(k % N1) * KS + (k / N1) * TL + l]; };
     // ---- outputs, stored from registers as they are formed ----------------
     // (row j of the line: synthesis F_j, j = 0..N; analysis S_j, j <= NYS)
     CT *Fo = nullptr;
@@ -445,7 +359,7 @@ k_ydct_r(Dims d, const double2 *__restrict__ roots, const double *__restrict__ c
     for (int c = 0; c < CH; ++c) {
         const int k = r * CH + c;
         if (k <= N / 2) {
-            const double2 zk = Z[k * TL + l], zm = Z[((N - k) % N) * TL + l];
+            const double2 zk = Z(k), zm = Z(k == 0 ? 0 : N - k);
             out(2 * k, cscale(0.5, cadd(zk, zm)));
             if (k >= 1 && k <= M) {
                 const double2 dz = csub(zk, zm);

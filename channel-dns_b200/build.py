@@ -6,12 +6,13 @@ The library lands beside the Python package: channel-dns_b200/cdns/libcdns_cuda.
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "cdns", "libcdns_cuda.so")
-SOURCES = ["context.cu", "chebyshev.cu", "transforms.cu", "solver.cu", "solver_setup.cu", "layout.cu", "noalloc.cu",
+SOURCES = ["context.cu", "chebyshev.cu", "transforms.cu", "any_length.cu", "solver.cu", "solver_setup.cu", "layout.cu", "noalloc.cu",
            "adjoint.cu", "adjoint_run.cu", "output.cu", "tune.cu",
            "field_files.cu", "pencil.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
@@ -35,16 +36,18 @@ def build(verbose: bool = False, extra=None) -> str:
         return OUT
     objdir = os.path.join(HERE, "_build")
     os.makedirs(objdir, exist_ok=True)
-    objs = []
-    for s in SOURCES:
-        obj = os.path.join(objdir, s.replace(".cu", ".o"))
+    def compile_one(src):
+        obj = os.path.join(objdir, src.replace(".cu", ".o"))
         cmd = [NVCC, *ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
-               "-I", os.path.join(ROOT, "include"), *FILE_FLAGS.get(s, []), *(extra or []),
-               "-c", os.path.join(CSRC, s), "-o", obj]
+               "-I", os.path.join(ROOT, "include"), *FILE_FLAGS.get(src, []), *(extra or []),
+               "-c", os.path.join(CSRC, src), "-o", obj]
         if verbose:
-            print(" ".join(cmd))
+            print(" ".join(cmd), flush=True)
         subprocess.run(cmd, check=True)
-        objs.append(obj)
+        return obj
+
+    with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+        objs = list(pool.map(compile_one, SOURCES))
     # the CUDA runtime is linked statically: the library always runs on the
     # runtime it was compiled against, whatever libcudart the host process loads
     cmd = [NVCC, *ARCH, "-shared", "-cudart", "static", "-o", OUT, *objs]

@@ -1,6 +1,7 @@
-// In-register DFTs for sm_100a: a length-N DFT (N <= 16) held by one thread,
+// In-register DFTs for sm_100a: a length-N DFT (N <= 25) held by one thread,
 // composed as N = A x B of the radix-2/3/4/5/7 butterflies of fft_lines.cuh
-// (unnormalised, FFTW sign convention: SIGN = -1 forward, +1 backward).
+// (A a butterfly, B a butterfly or composed itself; unnormalised, FFTW sign
+// convention: SIGN = -1 forward, +1 backward).
 // A length n = N1 x N2 transform then needs a single exchange through shared
 // memory between its two steps:
 //   step 1 (thread n2):  Y[k1] = W_n^(n2 k1) sum_n1 x[n2 + N2 n1] W_N1^(n1 k1)
@@ -11,11 +12,12 @@
 
 namespace cdns {
 
-// N = A x B with A, B in {1, 2, 3, 4, 5, 7}.
+// N = A x B with A in {2, 3, 4, 5, 7} and B = 1, one of them or a split length.
 template <int N> struct RegSplit;
 template <> struct RegSplit<2> { static constexpr int A = 2, B = 1; };
 template <> struct RegSplit<3> { static constexpr int A = 3, B = 1; };
 template <> struct RegSplit<4> { static constexpr int A = 4, B = 1; };
+template <> struct RegSplit<5> { static constexpr int A = 5, B = 1; };
 template <> struct RegSplit<6> { static constexpr int A = 2, B = 3; };
 template <> struct RegSplit<7> { static constexpr int A = 7, B = 1; };
 template <> struct RegSplit<8> { static constexpr int A = 2, B = 4; };
@@ -23,9 +25,15 @@ template <> struct RegSplit<9> { static constexpr int A = 3, B = 3; };
 template <> struct RegSplit<10> { static constexpr int A = 2, B = 5; };
 template <> struct RegSplit<12> { static constexpr int A = 3, B = 4; };
 template <> struct RegSplit<14> { static constexpr int A = 2, B = 7; };
+template <> struct RegSplit<15> { static constexpr int A = 3, B = 5; };
 template <> struct RegSplit<16> { static constexpr int A = 4, B = 4; };
+template <> struct RegSplit<18> { static constexpr int A = 2, B = 9; };
+template <> struct RegSplit<20> { static constexpr int A = 4, B = 5; };
+template <> struct RegSplit<21> { static constexpr int A = 3, B = 7; };
+template <> struct RegSplit<24> { static constexpr int A = 4, B = 6; };
+template <> struct RegSplit<25> { static constexpr int A = 5, B = 5; };
 
-// exp(-2 pi i k / N), N <= 16, as literals (cos and -sin of 2 pi k / N,
+// exp(-2 pi i k / N) as literals (cos and -sin of 2 pi k / N,
 // correctly rounded), so that twiddles that are the same in every lane need
 // no table loads.
 template <int N> __device__ __forceinline__ double2 kroot(int k);
@@ -105,6 +113,32 @@ template <> __device__ __forceinline__ double2 kroot<16>(int k) {
     return make_double2(c[k], s[k]);
 }
 
+template <> __device__ __forceinline__ double2 kroot<18>(int k) {
+    constexpr double c[18] = {1.0, 0.9396926207859084, 0.766044443118978, 0.5, 0.17364817766693036, -0.17364817766693036, -0.5, -0.766044443118978, -0.9396926207859084, -1.0, -0.9396926207859084, -0.766044443118978, -0.5, -0.17364817766693036, 0.17364817766693036, 0.5, 0.766044443118978, 0.9396926207859084};
+    constexpr double s[18] = {0.0, -0.3420201433256687, -0.6427876096865394, -0.8660254037844386, -0.984807753012208, -0.984807753012208, -0.8660254037844386, -0.6427876096865394, -0.3420201433256687, 0.0, 0.3420201433256687, 0.6427876096865394, 0.8660254037844386, 0.984807753012208, 0.984807753012208, 0.8660254037844386, 0.6427876096865394, 0.3420201433256687};
+    return make_double2(c[k], s[k]);
+}
+template <> __device__ __forceinline__ double2 kroot<20>(int k) {
+    constexpr double c[20] = {1.0, 0.9510565162951535, 0.8090169943749475, 0.5877852522924731, 0.30901699437494745, 0.0, -0.30901699437494745, -0.5877852522924731, -0.8090169943749475, -0.9510565162951535, -1.0, -0.9510565162951535, -0.8090169943749475, -0.5877852522924731, -0.30901699437494745, 0.0, 0.30901699437494745, 0.5877852522924731, 0.8090169943749475, 0.9510565162951535};
+    constexpr double s[20] = {0.0, -0.30901699437494745, -0.5877852522924731, -0.8090169943749475, -0.9510565162951535, -1.0, -0.9510565162951535, -0.8090169943749475, -0.5877852522924731, -0.30901699437494745, 0.0, 0.30901699437494745, 0.5877852522924731, 0.8090169943749475, 0.9510565162951535, 1.0, 0.9510565162951535, 0.8090169943749475, 0.5877852522924731, 0.30901699437494745};
+    return make_double2(c[k], s[k]);
+}
+template <> __device__ __forceinline__ double2 kroot<21>(int k) {
+    constexpr double c[21] = {1.0, 0.9555728057861407, 0.8262387743159949, 0.6234898018587335, 0.36534102436639504, 0.07473009358642425, -0.2225209339563144, -0.5, -0.7330518718298263, -0.9009688679024191, -0.9888308262251285, -0.9888308262251285, -0.9009688679024191, -0.7330518718298263, -0.5, -0.2225209339563144, 0.07473009358642425, 0.36534102436639504, 0.6234898018587335, 0.8262387743159949, 0.9555728057861407};
+    constexpr double s[21] = {0.0, -0.2947551744109042, -0.5633200580636221, -0.7818314824680298, -0.9308737486442042, -0.9972037971811801, -0.9749279121818236, -0.8660254037844386, -0.6801727377709194, -0.4338837391175581, -0.14904226617617444, 0.14904226617617444, 0.4338837391175581, 0.6801727377709194, 0.8660254037844386, 0.9749279121818236, 0.9972037971811801, 0.9308737486442042, 0.7818314824680298, 0.5633200580636221, 0.2947551744109042};
+    return make_double2(c[k], s[k]);
+}
+template <> __device__ __forceinline__ double2 kroot<24>(int k) {
+    constexpr double c[24] = {1.0, 0.9659258262890683, 0.8660254037844386, 0.7071067811865476, 0.5, 0.25881904510252074, 0.0, -0.25881904510252074, -0.5, -0.7071067811865476, -0.8660254037844386, -0.9659258262890683, -1.0, -0.9659258262890683, -0.8660254037844386, -0.7071067811865476, -0.5, -0.25881904510252074, 0.0, 0.25881904510252074, 0.5, 0.7071067811865476, 0.8660254037844386, 0.9659258262890683};
+    constexpr double s[24] = {0.0, -0.25881904510252074, -0.5, -0.7071067811865476, -0.8660254037844386, -0.9659258262890683, -1.0, -0.9659258262890683, -0.8660254037844386, -0.7071067811865476, -0.5, -0.25881904510252074, 0.0, 0.25881904510252074, 0.5, 0.7071067811865476, 0.8660254037844386, 0.9659258262890683, 1.0, 0.9659258262890683, 0.8660254037844386, 0.7071067811865476, 0.5, 0.25881904510252074};
+    return make_double2(c[k], s[k]);
+}
+template <> __device__ __forceinline__ double2 kroot<25>(int k) {
+    constexpr double c[25] = {1.0, 0.9685831611286311, 0.8763066800438636, 0.7289686274214116, 0.5358267949789967, 0.30901699437494745, 0.06279051952931337, -0.18738131458572463, -0.42577929156507266, -0.6374239897486897, -0.8090169943749475, -0.9297764858882515, -0.9921147013144779, -0.9921147013144779, -0.9297764858882515, -0.8090169943749475, -0.6374239897486897, -0.42577929156507266, -0.18738131458572463, 0.06279051952931337, 0.30901699437494745, 0.5358267949789967, 0.7289686274214116, 0.8763066800438636, 0.9685831611286311};
+    constexpr double s[25] = {0.0, -0.2486898871648548, -0.48175367410171527, -0.6845471059286887, -0.8443279255020151, -0.9510565162951535, -0.9980267284282716, -0.9822872507286887, -0.9048270524660196, -0.7705132427757893, -0.5877852522924731, -0.368124552684678, -0.12533323356430426, 0.12533323356430426, 0.368124552684678, 0.5877852522924731, 0.7705132427757893, 0.9048270524660196, 0.9822872507286887, 0.9980267284282716, 0.9510565162951535, 0.8443279255020151, 0.6845471059286887, 0.48175367410171527, 0.2486898871648548};
+    return make_double2(c[k], s[k]);
+}
+
 // v * exp(SIGN 2 pi i k / N) with the literal root: the exact cases (+-1, +-i)
 // fold to sign changes and swaps after unrolling; FP32 adds the product by the
 // rounding residue of the constant (the exact DFT up to arithmetic rounding).
@@ -150,7 +184,7 @@ __device__ __forceinline__ void dft_reg(C (&v)[N], const Twiddles<C> &, int) {
             C t[B];
 #pragma unroll
             for (int b = 0; b < B; ++b) t[b] = y[b * A + c];
-            bfly<B, SIGN>(t, static_cast<const C *>(nullptr), 0);
+            dft_reg<B, SIGN>(t, Twiddles<C>{nullptr, nullptr}, 0);
 #pragma unroll
             for (int d = 0; d < B; ++d) v[c + A * d] = t[d];
         }

@@ -105,5 +105,14 @@ template <class CT> struct YdctArgs {
     double inE = 1.0, inI = 1.0, s0 = 0.0, sk = 0.0;       // analysis weights and scales
 };
 
+// ---- any_length.cu: lengths n = N1 x N2 by factors switched at run time ----
+bool any_length(int n);
+cudaError_t configure_any_kernels(const Dims &d);
+// false (nothing launched) where the length has no such split
+bool launch_z_any(const Dims &d, const double2 *roots, const double2 *in, double2 *out, int nf, bool backward,
+                  int lines, bool coarse, cudaStream_t s);
+bool launch_x_cross_any(const Dims &d, const double2 *roots, const double2 *G, double2 *H, cudaStream_t s);
+template <class CT>
+bool launch_ydct_any(const Dims &d, const Tables &t, int nf, bool ana, const YdctArgs<CT> &A, cudaStream_t s);
 
 }  // namespace cdns

@@ -1671,6 +1671,8 @@ cudaError_t configure_transform_kernels(const Dims &d) {
     if (e != cudaSuccess) return e;
     e = configure_register_forms<float2>(d);
     if (e != cudaSuccess) return e;
+    e = configure_any_kernels(d);
+    if (e != cudaSuccess) return e;
     e = raise_smem(k_z_backward, (int)smem_zfft(widest_lines(d)));
     if (e != cudaSuccess) return e;
     e = raise_smem(k_z_forward, (int)smem_zfft(widest_lines(d)));
@@ -1764,6 +1766,7 @@ void launch_z_backward(const Dims &d, const FftPlan &P, const double2 *roots, co
                        double2 *G, int nf, cudaStream_t s, bool coarse) {
     if (z_backward_r(d, roots, F, G, nf, s, coarse)) return;
     const int tl = z_lines(d);
+    if (launch_z_any(d, roots, F, G, nf, true, tl, coarse, s)) return;
     dim3 grid((d.nkx + tl - 1) / tl, d.ny2, nf);
     k_z_backward<<<grid, 256, smem_zfft(d), s>>>(d, P, roots, F, G, tl, coarse);
 }
@@ -1771,6 +1774,7 @@ void launch_z_backward(const Dims &d, const FftPlan &P, const double2 *roots, co
 void launch_x_cross(const Dims &d, const FftPlan &P, const double2 *roots, const double2 *G,
                     double2 *H, cudaStream_t s) {
     if (x_cross_r<double2, false>(d, roots, G, H, nullptr, s)) return;
+    if (launch_x_cross_any(d, roots, G, H, s)) return;
     dim3 grid((d.NZ2 + kRW - 1) / kRW, d.ny2);
     k_x_cross<<<grid, 256, smem_xcross(d), s>>>(d, P, roots, G, H, kRW);
 }
@@ -1779,6 +1783,7 @@ void launch_z_forward(const Dims &d, const FftPlan &P, const double2 *roots, con
                       double2 *F, int nf, cudaStream_t s, bool coarse) {
     if (z_forward_r(d, roots, H, F, nf, s, coarse)) return;
     const int tl = z_lines(d);
+    if (launch_z_any(d, roots, H, F, nf, false, tl, coarse, s)) return;
     dim3 grid((d.nkx + tl - 1) / tl, d.ny2, nf);
     k_z_forward<<<grid, 256, smem_zfft(d), s>>>(d, P, roots, H, F, tl, coarse);
 }
@@ -1808,7 +1813,7 @@ void launch_x_adjoint(const Dims &d, const FftPlan &P, const double2 *roots, con
 }
 
 bool ydct_available(const Dims &d, const Tables &t) {
-    return t.root_y && d.NY2 % 2 == 0 && with_xsplit(d.NY2, [](auto, auto) {});
+    return t.root_y && d.NY2 % 2 == 0 && (with_xsplit(d.NY2, [](auto, auto) {}) || any_length(d.NY2));
 }
 
 template <class CT>
@@ -1816,7 +1821,7 @@ bool ydct(const Dims &d, const Tables &t, int nf, bool ana, const YdctArgs<CT> &
     if (!ydct_available(d, t)) return false;
     const int tl = ydct_lines(d);
     dim3 grid((d.nkx + tl - 1) / tl, d.nkz, nf);
-    return with_xsplit(d.NY2, [&](auto a, auto b) {
+    const bool reg = with_xsplit(d.NY2, [&](auto a, auto b) {
         constexpr int N1 = decltype(a)::value, N2 = decltype(b)::value;
         with_ydct_lines(tl, [&](auto w) {
             constexpr int TL = decltype(w)::value;
@@ -1827,6 +1832,7 @@ bool ydct(const Dims &d, const Tables &t, int nf, bool ana, const YdctArgs<CT> &
                 k_ydct_r<N1, N2, false, TL, CT><<<grid, 16 * TL, sm, s>>>(d, t.root_y, t.cosy, A);
         });
     });
+    return reg || launch_ydct_any(d, t, nf, ana, A, s);
 }
 bool launch_ydct(const Dims &d, const Tables &t, const double2 *src0, const double2 *src1, int nsplit, int nf,
                  double2 *out, bool ana, cudaStream_t s) {

@@ -165,6 +165,7 @@ int load_checkpoint(cdns_ctx *c, size_t i) {
     const size_t n3 = 3 * (size_t)d.Ns;
     const double2 *b = c->adj->ck + i * ck_size(d);
     c->cur = 0;
+    c->om_current = false;
     CK(cudaMemcpyAsync(c->U[0], b, n3 * sizeof(double2), cudaMemcpyDeviceToDevice, c->stream));
     CK(cudaMemcpyAsync(c->U[1], b + n3, n3 * sizeof(double2), cudaMemcpyDeviceToDevice, c->stream));
     CK(cudaMemcpyAsync(c->Nb[1], b + 2 * n3, n3 * sizeof(double2), cudaMemcpyDeviceToDevice, c->stream));
@@ -182,7 +183,7 @@ void forward_step(cdns_ctx *c, int it, const SolverState &st, double2 *G, bool s
     const int k = c->cur;
     const Dims &d = c->d;
     if (!solve) {
-        launch_curl(d, c->t, c->U[k], c->om, nullptr, c->pp.Re, c->stream);
+        ensure_curl(c);
         launch_ysynth(d, c->t, c->U[k], c->om, 3, 6, c->F, c->stream);
         launch_z_backward(d, c->pz, c->t.root_z, c->F, G, 6, c->stream);
         return;
@@ -193,7 +194,7 @@ void forward_step(cdns_ctx *c, int it, const SolverState &st, double2 *G, bool s
     a.u_prev = c->U[1 - k];
     a.N = c->Nb[k];
     a.N_prev = c->Nb[1 - k];
-    a.bw = c->bw;
+    a.bw = c->bwb[k];
     a.B_prev = c->Bb[1 - k];
     a.B_new = c->Bb[k];
     a.bc_v = c->bc_v;
@@ -205,7 +206,10 @@ void forward_step(cdns_ctx *c, int it, const SolverState &st, double2 *G, bool s
     a.a1 = a1;
     a.b0 = b0;
     a.b1 = b1;
+    a.om = c->om;
+    a.bw_out = c->bwb[1 - k];
     launch_step_solve(c->d, c->t, c->pp, g, st, a, c->stream);
+    c->om_current = true;
     c->cur = 1 - k;
 }
 

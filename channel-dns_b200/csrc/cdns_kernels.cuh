@@ -151,6 +151,8 @@ struct StepArgs {
     double a0, a1, b0, b1;
     const double2 *bc_p;        // if set: pressure wall data [2][ncol] used as is
     int solve_only;             // 1: solve_modes alone (no zero-mode / flow correction)
+    double2 *om;                // if set: the curl of u_out [3][Ns] and its pressure-wall sums
+    double2 *bw_out;            // [2][ncol]
 };
 
 // ---- solver_setup.cu ----

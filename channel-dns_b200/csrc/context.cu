@@ -82,6 +82,13 @@ void step_coefficients(int it, double dt, double re, double &a0, double &a1, dou
     g = (a0 + a1) * re;
 }
 
+void ensure_curl(cdns_ctx *c) {
+    c->bw = c->bwb[c->cur];
+    if (c->om_current) return;
+    launch_curl(c->d, c->t, c->U[c->cur], c->om, c->bw, c->pp.Re, c->stream);
+    c->om_current = true;
+}
+
 void enqueue_nonlinear(cdns_ctx *c, const double2 *u, double2 *N, bool prof, int step_slot, double2 *G_fp64) {
     const Dims &d = c->d;
     cudaStream_t s = c->stream;
@@ -89,7 +96,13 @@ void enqueue_nonlinear(cdns_ctx *c, const double2 *u, double2 *N, bool prof, int
         if (prof) cudaEventRecord(c->ev[(size_t)step_slot * (kStages + 1) + stage], s);
     };
     mark(0);
-    launch_curl(d, c->t, u, c->om, c->bw, c->pp.Re, s);
+    if (u == c->U[c->cur]) {
+        ensure_curl(c);
+    } else {
+        c->bw = c->bwb[c->cur];
+        launch_curl(d, c->t, u, c->om, c->bw, c->pp.Re, s);
+        c->om_current = false;
+    }
     mark(1);
     if (c->mixed) {
         float2 *F = reinterpret_cast<float2 *>(c->F), *G = reinterpret_cast<float2 *>(c->G);
@@ -130,7 +143,7 @@ void enqueue_solve(cdns_ctx *c, double a0, double a1, double b0, double b1, doub
     a.u_prev = c->U[1 - k];
     a.N = c->Nb[k];
     a.N_prev = c->Nb[1 - k];
-    a.bw = c->bw;
+    a.bw = c->bwb[k];
     a.B_prev = c->Bb[1 - k];
     a.B_new = c->Bb[k];
     a.bc_v = c->bc_v;
@@ -142,7 +155,10 @@ void enqueue_solve(cdns_ctx *c, double a0, double a1, double b0, double b1, doub
     a.a1 = a1;
     a.b0 = b0;
     a.b1 = b1;
+    a.om = c->om;
+    a.bw_out = c->bwb[1 - k];
     launch_step_solve(c->d, c->t, c->pp, g_v, c->st, a, c->stream);
+    c->om_current = true;   // of u_out, the current velocity once the caller rotates
 }
 
 int require_whole(const cdns_ctx *c) {
@@ -185,6 +201,7 @@ int one_step(cdns_ctx *c, int it) {
         int r = do_setup(c, g);
         if (r) return r;
     }
+    ensure_curl(c);
     if (c->prof) {
         if (c->prof_steps >= kMaxProfSteps) return fail(CDNS_ERR_STATE, "profiling window full");
         enqueue_step_body(c, a0, a1, b0, b1, g, true, c->prof_steps);
@@ -359,7 +376,7 @@ int create_context(const cdns_mesh_desc *m, const cdns_params *p, int precision,
     if ((r = c->alloc(c->U[0], 3 * Ns)) || (r = c->alloc(c->U[1], 3 * Ns)) ||
         (r = c->alloc(c->Nb[0], 3 * Ns)) || (r = c->alloc(c->Nb[1], 3 * Ns)) ||
         (r = c->alloc(c->Bb[0], 2 * nc)) || (r = c->alloc(c->Bb[1], 2 * nc)) ||
-        (r = c->alloc(c->p, Ns)) || (r = c->alloc(c->bw, 2 * nc)) || (r = c->alloc(c->bc_v, 6 * nc)) ||
+        (r = c->alloc(c->p, Ns)) || (r = c->alloc(c->bwb[0], 2 * nc)) || (r = c->alloc(c->bwb[1], 2 * nc)) || (r = c->alloc(c->bc_v, 6 * nc)) ||
         (r = c->alloc(c->bc_p, 2 * nc)) || (r = c->alloc(c->F, fbuf)) || (r = c->alloc(c->G, gbuf)) ||
         (r = c->alloc(c->H, hbuf)) || (r = c->alloc(c->aux, 3 * Ns)) || (r = c->alloc(c->aux2, 3 * Ns)) ||
         (r = c->alloc(c->zero3, 3 * Ns)) || (r = c->alloc(c->om, 3 * Ns)) ||
@@ -367,6 +384,7 @@ int create_context(const cdns_mesh_desc *m, const cdns_params *p, int precision,
         (r = c->alloc(c->phys, (size_t)d.NZ2 * d.ny2 * d.NX2)) || (r = c->alloc(c->dpdx, 2)) ||
         (r = c->alloc(c->err, 1)))
         return bail(r);
+    c->bw = c->bwb[0];
     SolverState &st = c->st;
     if ((r = c->alloc(st.wn_p, nc)) || (r = c->alloc(st.wn_v, nc)) || (r = c->alloc(st.ad_p, Ns)) ||
         (r = c->alloc(st.ad_v, Ns)) || (r = c->alloc(st.p_inf, 2 * Ns)) || (r = c->alloc(st.v_inf, 6 * Ns)) ||
@@ -426,6 +444,7 @@ int cdns_set_velocity_device(cdns_ctx *c, const double *v) {
     DeviceGuard guard(c->device);
     const Dims &d = c->d;
     c->cur = 0;
+    c->om_current = false;
     launch_deinterleave(reinterpret_cast<const double2 *>(v), c->U[0], d.Ns, 3, c->stream);
     CK(cudaMemsetAsync(c->U[1], 0, sizeof(double2) * 3 * d.Ns, c->stream));
     CK(cudaMemsetAsync(c->Nb[0], 0, sizeof(double2) * 3 * d.Ns, c->stream));
@@ -454,6 +473,7 @@ int cdns_update_velocity(cdns_ctx *c, const double *v) {
     DeviceGuard guard(c->device);
     CK(cudaMemcpyAsync(c->aux, v, sizeof(double2) * 3 * c->d.Ns, cudaMemcpyHostToDevice, c->stream));
     // the current slot only: u_prev, N_prev and B_prev of the multistep history stay
+    c->om_current = false;
     launch_deinterleave(reinterpret_cast<const double2 *>(c->aux), c->U[c->cur], c->d.Ns, 3, c->stream);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->stream));
@@ -840,6 +860,7 @@ int batch_step(cdns_batch *b, int it) {
         }
         return CDNS_OK;
     }
+    for (cdns_ctx *m : b->members) ensure_curl(m);
     cudaGraphExec_t &ge = b->graph[b->members[0]->cur];
     if (!ge) {
         cudaGraph_t graph;

@@ -61,9 +61,12 @@ struct cdns_ctx {
     double2 *Nb[2] = {nullptr, nullptr};  // nonlinear term, current / previous
     double2 *Bb[2] = {nullptr, nullptr};  // pressure wall data, current / previous
     int cur = 0;                          // U[cur] = u, Nb[cur] = next N, Bb[cur] = next B
-    double2 *p = nullptr, *bw = nullptr, *bc_v = nullptr, *bc_p = nullptr;
+    double2 *p = nullptr, *bc_v = nullptr, *bc_p = nullptr;
+    double2 *bwb[2] = {nullptr, nullptr}; // vorticity part of the pressure wall data, bwb[cur] of U[cur]
+    double2 *bw = nullptr;                // ... of the last nonlinear evaluation (one of the two)
     double2 *F = nullptr, *G = nullptr, *H = nullptr, *aux = nullptr, *aux2 = nullptr, *zero3 = nullptr;
     double2 *om = nullptr;                // vorticity of the velocity being transformed
+    bool om_current = false;              // om and bwb[cur] belong to U[cur] (the solve leaves them so)
     bool mixed = false;                   // FP32 fine-grid stages (CDNS_PRECISION_MIXED)
     double *mean = nullptr;               // mixed: FP64 (kz, kx) = (0, 0) profiles [6][NY2+1]
     double *phys = nullptr;
@@ -110,6 +113,9 @@ namespace cdns {
 // Multistep coefficients of iteration it (src/sim/simulation.cpp:36-45).
 void step_coefficients(int it, double dt, double re, double &a0, double &a1, double &b0, double &b1,
                        double &g);
+// om and bwb[cur] of the current velocity: the last solve left them, unless the
+// velocity or om changed since.  Called before a step is enqueued or replayed.
+void ensure_curl(cdns_ctx *c);
 // Nonlinear stages u -> N (planar spectral) and bw; G_fp64 (FP64 contexts)
 // receives the z-physical fields of u and omega, c->G if null.
 void enqueue_nonlinear(cdns_ctx *c, const double2 *u, double2 *N, bool prof, int step_slot,

@@ -400,7 +400,7 @@ int cdns_pencil_stage(cdns_ctx *c, int iteration, int stage) {
     if (stage == 0) {
         // EqSolvePV::setup at it = 1, 2 (src/sim/simulation.cpp:176-177)
         if ((r = do_setup(c, g))) return r;
-        launch_curl(d, c->t, c->U[k], c->om, c->bw, c->pp.Re, s);
+        ensure_curl(c);
         launch_ysynth(d, c->t, c->U[k], c->om, 3, 6, c->F, s);
         if (!w->peers) r = part_copy(w->block[0], w->chunk_max[0][0], true, c->F, w->buf[0][0], s);
     } else if (stage == 1) {

@@ -1,35 +1,51 @@
 // Per-(kz, kx) Chebyshev-tau pressure/velocity solve of the channel-dns step
 // (EqSolvePV, src/solver/eqsolve_pv.cpp) for sm_100a.
 //
-// One warp owns one spectral column (kz, kx) and keeps all its y coefficients
-// in registers.  Lane L = 2h + p holds, for every field, the coefficients of
-// parity p at y = 2(E h + e) + p, e = 0..E-1 (E = ceil((NYS+1)/32) rounded up
-// to 1, 2, 4 or 8).  Every tau recurrence (src/solver/eqsolve_pv.cpp:64-128)
-// and every Chebyshev derivative recurrence (src/solver/vector_ops.cpp:17-25)
-// couples only coefficients of one parity, so each becomes a first-order
-// affine recurrence along the 16 lanes of that parity: a sequential pass over
-// a lane's E coefficients, a 4-level shuffle scan over the lanes, and a
-// carry-in.  Wall sums are shuffle reductions.  This reassociates the
-// reference's sequential sums and recurrences; the results agree with the
-// sequential order to round-off (tested against the oracle at 1e-10).
+// Every tau recurrence (src/solver/eqsolve_pv.cpp:64-128) and every Chebyshev
+// derivative recurrence (src/solver/vector_ops.cpp:17-25) couples only
+// coefficients of one parity of y, and its multipliers are real: a column is
+// four independent scalar chains per field, (parity, re/im).  One thread runs
+// one chain sequentially, in the reference's order, over columns staged in
+// shared memory: a block holds TC consecutive columns, a warp the 4 TC chains of
+// one field, so that a row of the tile is read by 16 lanes as 128 consecutive
+// bytes.  The whole solve is two sweeps down and up the chain for the pressure
+// (one warp) and two for the velocity (three warps, one per component); the
+// right-hand sides (divergence of R, Re (grad P - R)) are formed inside the
+// downward sweep and the wall sums inside the upward one.
 //
-// The step solve reads the spectral state in its planar [kz][y][kx] layout
-// through swizzled shared-memory tiles (a block of TC warps owns TC
-// consecutive columns, so every global access is a coalesced row of TC
-// columns).  The warps leave the uncorrected solution in the tiles together
-// with four coefficients per column; the influence-matrix and sigma
-// corrections then run over the block as one coalesced elementwise pass over
-// the planar influence and B-problem fields (solver_setup.cu).  The tau
-// pivots are stored column-major ([col][y]) and read by each warp directly.
+// The influence-matrix and sigma corrections then run over the block as one
+// coalesced elementwise pass over the planar influence and B-problem fields
+// (solver_setup.cu).  Three symmetries cut what that pass reads from twelve
+// real fields to six over the kz <= 0 half:
+//   - the second influence response is the mirror image of the first under
+//     y -> -y (the wall conditions are the same on both sides): its pressure, u
+//     and w coefficients are (-1)^y times the first's, its v -(-1)^y times;
+//   - u and w are i kx phi and i kz phi of one phi where u and w have the same
+//     wall condition, so one of the two gives the other;
+//   - column -kz has the same pressure, u, v and pivots and w negated.
+// What bounds it: the chains' latency at 12 warps per SM against the streams
+// of the multistep state; blocks of kz and -kz run next to each other, so the
+// half fields are read from HBM once.
 #include "cdns_kernels.cuh"
 #include "warp_columns.cuh"
 
 namespace cdns {
 
 namespace {
-constexpr int TC = kColsPerBlock;     // columns (warps) per block
-constexpr int kThreads = 32 * TC;
+constexpr int TC = kColsPerBlock;     // columns per block
+constexpr int kThreads = 128;         // warp 0: pressure; warps 0-2: velocity; all: staging
+constexpr int kRowGroups = kThreads / TC;
 
+__device__ __forceinline__ double2 ld256(const double2 *p) {
+    double2 v;
+    asm("ld.global.L2::256B.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double ld256(const double *p) {
+    double v;
+    asm("ld.global.L2::256B.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
 struct SolveArgs {
     double p_a, p_b;           // pressure wall condition a P + b dP/dn
     double2 *p_out;            // [Ns] planar
@@ -37,335 +53,489 @@ struct SolveArgs {
     StepArgs step;
 };
 
+// Row stride of the staged pivots [TC][ncy]: = 2 (mod 16) doubles, so that the
+// chains of one warp (columns l, parities p: offset l stride + p) fall on
+// distinct banks.
+__host__ __device__ inline int pivot_stride(int ncy) { return ncy + ((2 - ncy % 16) + 16) % 16; }
 
-// Tau solve of (D^2 - k^2 - g) f = r with a f + b f' = (lower, upper) at
-// y = (+1, -1), both parities at once (src/solver/eqsolve_pv.cpp:64-128).
-// r must be zero beyond ny.  Returns false in a lane whose parity's pivot is
+// Rows of a chain that are worked on together.  One warp runs 32 chains, so a
+// chain costs what its instructions cost in sequence: a row has two dependent
+// operations of the recurrence (9 cycles each) and about 15 that do not depend
+// on it and overlap with those of the other rows of a group.
+constexpr int kRows = 4;
+
+// One chain of the tau solve of (D^2 - k^2 - g) f = r with a f + b f' =
+// (lower, upper) at y = (+1, -1): the coefficients of parity p of one scalar
+// part (re or im) of one column, in f[y * 2 TC].
+//   down  X_y = t_y - (WR w AD_{y+2}) X_{y+2},  t_y = WL r_{y-2} + WD r_y + WR r_{y+2},
+//         o = X_p - sum ad01_y AD_y X_y, ad01_{y-2} = tau(y-2) - (WL_y w AD_y) ad01_y
+//   up    Z_p = o / ad01_p,  Z_y = AD_y X_y - (WL_y w AD_y) Z_{y-2}
+// carried as g_y = AD_y X_y, which is what f holds between the sweeps.  As WD =
+// -(WL + WR) (half of WL at y = 2, where r_0 counts twice), t_y = WL D_y - WR
+// D_{y+2} with the differences D_y = r_{y-2} - r_y, D_2 = r_0 - r_2 / 2: a y
+// derivative in r then is a local term, 2 (y - 1) f_{y-1}, and needs no recurrence
+// of its own.  The two top rows, where the tau truncation drops terms, are written
+// out.  rhs.start(top) returns r_top; rhs.load(i, y) fetches the operands of row y
+// into slot i, rhs.diff(i, yd) returns D_y (yd = y, rows descending), rhs.diff2(i) D_2.
+// W[y] = (WL, WR).  acc(yd, Z_y) sees the solution.  Returns false if the pivot is
 // zero or not finite.
-template <int E>
-__device__ bool tau_warp(int ny, double g, double a, double b, bool zero_col, double2 lower,
-                         double2 upper, double w, const double2 (&r)[E], double2 (&out)[E],
-                         const double (&ad)[E], const double *__restrict__ WL,
-                         const double *__restrict__ WD, const double *__restrict__ WR) {
-    const int L = lane_id(), p = L & 1;
-    const bool normalize = g == 0.0 && a == 0.0 && zero_col;
+template <class Rhs, class Acc>
+__device__ __forceinline__ bool tau_chain(int ny, int p, double a, double b, bool normalize, double lower,
+                                          double upper, double w, const double2 *W,
+                                          const double *__restrict__ WD, const double *ad, double *f, Rhs &rhs,
+                                          Acc &&acc) {
     const int top = ((ny & 1) == p) ? ny : ny - 1;
-    double2 rr[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) rr[e] = r[e];
-    if (normalize) {
+    // diagonal of the boundary row, tau(y) = ta + tb y^2 (eqsolve_pv.cpp:64-70)
+    const bool dir = a == 0.0 && b == 0.0;
+    const double ta = dir ? (double)p : a, tb = dir ? (double)(1 - p) : b;
+    const double x0 = p ? (lower - upper) / 2.0 : (lower + upper) / 2.0;
+    const bool even_zero = normalize && p == 0;
+    double d2 = 0.0;
+    if (even_zero) {
         // the even chain of the singular zero column is closed by the mean
         // (eqsolve_pv.cpp:71-79): r_0 <- sum_{y>=2 even} r_y/(y^2-1) + (lo+up)/(2b)
-        double2 part = mk(0.0, 0.0);
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const int y = ycoef<E>(e);
-            if (p == 0 && y >= 2 && y <= ny) part = cadd(part, cdivr(r[e], (double)(y * y - 1)));
+        Rhs pre = rhs;
+        double r = pre.start(top), corr = 0.0;
+        for (int y = top; y >= 2; y -= 2) {
+            const double yq = (double)y;
+            corr += r / (yq * yq - 1.0);
+            if (y == 2) break;
+            pre.load(0, y);
+            r += pre.diff(0, yq);
         }
-        part = sum_parity(part);
-        if (b != 0.0) part = cadd(part, cdivr(cadd(lower, upper), 2.0 * b));
-        if (L == 0) rr[0] = part;
+        if (b != 0.0) corr += (lower + upper) / (2.0 * b);
+        d2 = corr - 0.5 * r;
     }
-    // three-term combination of the rhs
-    double2 rm2_0 = shfl2_up(rr[E - 1], 2);
-    double2 rp2_l = shfl2_down(rr[0], 2);
-    if (L + 2 >= 32) rp2_l = mk(0.0, 0.0);
-    double2 X[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const int y = ycoef<E>(e);
-        const double2 rm2 = e > 0 ? rr[(e + E - 1) % E] : rm2_0;
-        const double2 rp2 = e + 1 < E ? rr[(e + 1) % E] : rp2_l;
-        if (y > ny) X[e] = mk(0.0, 0.0);
-        else if (y == p) X[e] = (p == 0) ? cdivr(cadd(lower, upper), 2.0) : cdivr(csub(lower, upper), 2.0);
-        else if (y >= ny - 1) X[e] = cadd(cscale(WL[y], rm2), cscale(WD[y], rr[e]));
-        else X[e] = cadd(cadd(cscale(WL[y], rm2), cscale(WD[y], rr[e])), cscale(WR[y], rp2));
-    }
-    // pivots one step up the chain, AD(y + 2)
-    double adn_l = __shfl_down_sync(kFull, ad[0], 2);
-    if (L + 2 >= 32) adn_l = 0.0;
-    // backward sweep X_y -= (WR_y w AD_{y+2}) X_{y+2} for 2 <= y <= top - 2
-    double A[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const int y = ycoef<E>(e);
-        const double adn = e + 1 < E ? ad[(e + 1) % E] : adn_l;
-        A[e] = (y >= 2 && y <= top - 2) ? -((WR[y] * w) * adn) : 0.0;
-    }
-    affine_suffix<E>(A, X);
-    // pivot chain ad01_j = tau(j) - (WL_{j+2} w ad01_{j+2}) AD_{j+2}, ad01_top = tau(top)
-    double Aa[E], Ba[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const int y = ycoef<E>(e);
-        const double adn = e + 1 < E ? ad[(e + 1) % E] : adn_l;
-        if (y > top) {
-            Aa[e] = 0.0;
-            Ba[e] = 0.0;
-        } else if (y == top) {
-            Aa[e] = 0.0;
-            Ba[e] = tau_func(a, b, y);
-        } else {
-            Aa[e] = -((WL[y + 2] * w) * adn);
-            Ba[e] = tau_func(a, b, y);
+    double yd = (double)top, ad01 = ta + tb * (yd * yd), g = 0.0, o = 0.0, dup = 0.0;   // dup = D_{y+2}
+    // one row: g_y from t_y; the boundary sum and its next multiplier
+    auto row = [&](int y, double t, double av, double2 wy) {
+        const double wa = w * av;
+        g = av * t - (wa * wy.y) * g;
+        o += ad01 * g;
+        yd -= 2.0;
+        ad01 = (ta + tb * (yd * yd)) - (wa * wy.x) * ad01;
+        f[y * (2 * TC)] = g;
+    };
+    int y = top;
+    {
+        const double r0 = rhs.start(top);
+        rhs.load(0, y);
+        const double dt = rhs.diff(0, yd), r1 = dt + r0;   // r_{top-2}
+        row(y, W[y].x * r1, ad[y], W[y]);
+        y -= 2;
+        if (y >= 2) {
+            rhs.load(0, y);
+            dup = y > 2 ? rhs.diff(0, yd) : even_zero ? d2 : rhs.diff2(0);
+            row(y, W[y].x * (dup + (y > 2 ? r1 : 0.5 * r1)) + WD[y] * r1, ad[y], W[y]);
+            y -= 2;
         }
     }
-    affine_suffix<E>(Aa, Ba);
-    // o0 = X_par - sum_{j = par+2..top} ad01_j AD_j X_j ; pivot ad01_par
-    double2 s = mk(0.0, 0.0);
+    for (; y - 2 * (kRows - 1) >= 3; y -= 2 * kRows) {
+        double av[kRows], t[kRows];
+        double2 wy[kRows];
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const int y = ycoef<E>(e);
-        if (y >= p + 2 && y <= top) s = cadd(s, cscale(Ba[e] * ad[e], X[e]));
-    }
-    s = sum_parity(s);
-    double2 o0 = csub(shfl2(X[0], p), s);
-    double piv = __shfl_sync(kFull, Ba[0], p);
-    if (normalize && p == 0) {
-        o0 = mk(0.0, 0.0);
-        piv = 1.0;
-    }
-    const bool ok = isfinite(piv) && piv != 0.0;
-    const double2 zpar = cdivr(o0, piv);
-    // forward sweep Z_y = AD_y (X_y - WL_y w Z_{y-2})
+        for (int i = 0; i < kRows; ++i) {
+            rhs.load(i, y - 2 * i);
+            wy[i] = W[y - 2 * i];
+            av[i] = ad[y - 2 * i];
+        }
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const int y = ycoef<E>(e);
-        if (y == p) {
-            A[e] = 0.0;
-            X[e] = zpar;
-        } else if (y <= ny) {
-            A[e] = -(ad[e] * (WL[y] * w));
-            X[e] = cscale(ad[e], X[e]);
-        } else {
-            A[e] = 0.0;
-            X[e] = mk(0.0, 0.0);
+        for (int i = 0; i < kRows; ++i) {
+            const double dq = rhs.diff(i, yd - (double)(2 * i));
+            t[i] = wy[i].x * dq - wy[i].y * dup;
+            dup = dq;
+        }
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) row(y - 2 * i, t[i], av[i], wy[i]);
+    }
+    for (; y >= 2; y -= 2) {
+        rhs.load(0, y);
+        const double2 wy = W[y];
+        const double dq = y > 2 ? rhs.diff(0, yd) : even_zero ? d2 : rhs.diff2(0);
+        row(y, wy.x * dq - wy.y * dup, ad[y], wy);
+        dup = dq;
+    }
+    double z = x0 - o;
+    if (even_zero) {
+        z = 0.0;
+        ad01 = 1.0;
+    }
+    const bool ok = isfinite(ad01) && ad01 != 0.0;
+    z /= ad01;
+    f[p * (2 * TC)] = z;
+    yd = (double)p;
+    acc(yd, z);
+    y = p + 2;
+    for (; y + 2 * (kRows - 1) <= ny; y += 2 * kRows) {
+        double gv[kRows], n[kRows];
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            gv[i] = f[(y + 2 * i) * (2 * TC)];
+            n[i] = W[y + 2 * i].x * (w * ad[y + 2 * i]);
+        }
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            z = gv[i] - n[i] * z;
+            f[(y + 2 * i) * (2 * TC)] = z;
+            yd += 2.0;
+            acc(yd, z);
         }
     }
-    affine_prefix<E>(A, X);
-#pragma unroll
-    for (int e = 0; e < E; ++e) out[e] = ycoef<E>(e) <= ny ? X[e] : mk(0.0, 0.0);
+    for (; y <= ny; y += 2) {
+        z = f[y * (2 * TC)] - (W[y].x * (w * ad[y])) * z;
+        f[y * (2 * TC)] = z;
+        yd += 2.0;
+        acc(yd, z);
+    }
     return ok;
 }
 
-template <int E>
-__global__ void __launch_bounds__(kThreads, E <= 4 ? 2 : 1)
+// Right-hand side of the pressure: the divergence of R, q + dR_1/dy with q =
+// i kx R_0 + i kz R_2 (src/solver/eqsolve_pv.cpp:340-357).  own / other: this
+// thread's part of the column and the other one (i k swaps re and im; sx, sz
+// carry the sign).
+struct DivergenceRhs {
+    const double *r0_other, *r1_own, *r2_other;
+    double sx, sz;
+    int ny;
+    double q = 0.0, a0[kRows], a1[kRows], a2[kRows];
+    __device__ __forceinline__ double start(int top) {
+        q = sx * r0_other[top * (2 * TC)] + sz * r2_other[top * (2 * TC)];
+        return top < ny ? q + (2.0 * ny) * r1_own[ny * (2 * TC)] : q;
+    }
+    __device__ __forceinline__ void load(int i, int y) {
+        a0[i] = r0_other[(y - 2) * (2 * TC)];
+        a2[i] = r2_other[(y - 2) * (2 * TC)];
+        a1[i] = r1_own[(y - 1) * (2 * TC)];
+    }
+    __device__ __forceinline__ double diff(int i, double yd) {
+        const double qn = sx * a0[i] + sz * a2[i], d = (qn - q) + (2.0 * yd - 2.0) * a1[i];
+        q = qn;
+        return d;
+    }
+    __device__ __forceinline__ double diff2(int i) { return (sx * a0[i] + sz * a2[i] - 0.5 * q) + a1[i]; }
+};
+
+// Right-hand side of velocity component C: Re (grad P - R_C)
+// (src/solver/eqsolve_pv.cpp:359-395); pp: P's own part for C = 1, else the other one.
+template <int C> struct VelocityRhs {
+    const double *pp, *r_own;
+    double s_i, re;
+    int ny;
+    double q = 0.0, a[kRows], r[kRows];   // q: C = 1: -Re R_1, else the whole r_y
+    __device__ __forceinline__ double start(int top) {
+        if (C == 1) {
+            q = -re * r_own[top * (2 * TC)];
+            return top < ny ? q + re * ((2.0 * ny) * pp[ny * (2 * TC)]) : q;
+        }
+        q = re * (s_i * pp[top * (2 * TC)] - r_own[top * (2 * TC)]);
+        return q;
+    }
+    __device__ __forceinline__ void load(int i, int y) {
+        r[i] = r_own[(y - 2) * (2 * TC)];
+        a[i] = pp[(C == 1 ? y - 1 : y - 2) * (2 * TC)];
+    }
+    __device__ __forceinline__ double diff(int i, double yd) {
+        double d;
+        if (C == 1) {
+            const double qn = -re * r[i];
+            d = (qn - q) + (re * (2.0 * yd - 2.0)) * a[i];
+            q = qn;
+        } else {
+            const double qn = re * (s_i * a[i] - r[i]);
+            d = qn - q;
+            q = qn;
+        }
+        return d;
+    }
+    __device__ __forceinline__ double diff2(int i) {
+        if (C == 1) return (-re * r[i] - 0.5 * q) + re * a[i];
+        return re * (s_i * a[i] - r[i]) - 0.5 * q;
+    }
+};
+
+__global__ void __launch_bounds__(kThreads, 3)
 k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A) {
-    extern __shared__ double2 tile[];   // [4][ncy][TC]
-    __shared__ double2 s_c0[TC], s_c1[TC], s_sg[2][TC];   // per-column correction coefficients
+    extern __shared__ double2 tile[];   // [4][ncy][TC]: R_0, R_1, R_2, P; then (WL, WR) and the pivots
+    __shared__ double s_wall[3][2][2 * TC];
+    __shared__ double2 s_cs[TC], s_cd[TC], s_sg[2][TC];   // c0 + c1, c0 - c1, sigma
     const int ncy = d.ncy, ny = d.NYS, nkx = d.nkx, ncol = d.ncol;
     const int S = ncy * TC;
-    const int col0 = blockIdx.x * TC;
+    const int AS = pivot_stride(ncy);
+    double2 *s_w = tile + 3 * S + max(ncy, kRowGroups) * TC;         // [ncy] (WL, WR)
+    double *s_ad = reinterpret_cast<double *>(s_w + ncy);             // [TC][AS]
+    // blocks of kz and -kz next to each other: from both ends inwards
+    const int blk = (blockIdx.x & 1) ? (int)gridDim.x - 1 - (int)(blockIdx.x >> 1) : (int)(blockIdx.x >> 1);
+    const int col0 = blk * TC;
     const int tid = threadIdx.x;
-    const int w = tid >> 5;
-    const int L = tid & 31, p = L & 1;
-    const int col = col0 + w;
+    const int w = tid >> 5, lane = tid & 31;
     const StepArgs &s = A.step;
 
-    // ---- stage R = a0 u + a1 u_prev + b0 N + b1 N_prev and N_y -------------
-#pragma unroll 2
-    for (int i = tid; i < S; i += kThreads) {
-        const int y = i / TC, l = i - (i / TC) * TC;
-        const int c2 = col0 + l;
-        if (c2 < ncol) {
-            const int kzi = c2 / nkx, kx = c2 - (c2 / nkx) * nkx;
-            const long long off = ((long long)kzi * ncy + y) * nkx + kx;
-            const int sl = tile_slot<E>(y, l);
-            double2 nv[3];
+    // this thread's column in the row-wise passes: l = tid mod TC, rows g, g + 16, ...
+    const int l = tid & (TC - 1), g = tid / TC;
+    const int c2 = col0 + l;
+    const bool ok = c2 < ncol;
+    const int kzi = ok ? c2 / nkx : 0, kx = ok ? c2 - kzi * nkx : 0;
+    const int kzn = kzi <= d.NZS ? kzi : 2 * d.NZS - kzi;   // the kz <= 0 column of this |kz|
+
+    // ---- pivots of the kz <= 0 columns (column-major) and the row weights ---
+    auto pivot_base = [&](int q) {
+        const int c = min(col0 + q, ncol - 1), kq = c / nkx;
+        return (long long)(min(kq, 2 * d.NZS - kq) * nkx + (c - kq * nkx)) * ncy;
+    };
+    for (int q = w; q < TC; q += kThreads / 32) {
+        const double *src = st.ad_p + pivot_base(q);
+        for (int y = lane; y < ncy; y += 32) cp_async8(s_ad + q * AS + y, src + y, 8);
+    }
+    for (int y = tid; y < ncy; y += kThreads) {
+        cp_async8(&s_w[y].x, t.WL + y, 8);
+        cp_async8(&s_w[y].y, t.WR + y, 8);
+    }
+    cp_async_commit();
+
+    // ---- stage R = a0 u + a1 u_prev + b0 N + b1 N_prev; sums of N_y --------
+    // (the loads of two rows are issued before the first use)
+    {
+        constexpr int kBatch = 2;
+        double2 sy = mk(0.0, 0.0);   // N_y over this thread's rows (all of parity g & 1)
+        const long long base = (long long)kzi * ncy * nkx + kx;
+        for (int y0 = g; ok && y0 < ncy; y0 += kBatch * kRowGroups) {
+            double2 u[kBatch][3], up[kBatch][3], nv[kBatch][3], np[kBatch][3];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const long long o = c * d.Ns + off;
-                nv[c] = s.N[o];
-                // R (src/sim/simulation.cpp:151-158)
-                tile[c * S + sl] = cadd(cadd(cadd(cscale(s.a0, s.u[o]), cscale(s.a1, s.u_prev[o])),
-                                             cscale(s.b0, nv[c])),
-                                        cscale(s.b1, s.N_prev[o]));
+            for (int b = 0; b < kBatch; ++b) {
+                const int y = min(y0 + b * kRowGroups, ny);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const long long o = c * d.Ns + base + (long long)y * nkx;
+                    u[b][c] = ld256(s.u + o);
+                    up[b][c] = ld256(s.u_prev + o);
+                    nv[b][c] = ld256(s.N + o);
+                    np[b][c] = ld256(s.N_prev + o);
+                }
             }
-            tile[3 * S + sl] = nv[1];
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b) {
+                const int y = y0 + b * kRowGroups;
+                if (y >= ncy) break;
+#pragma unroll
+                for (int c = 0; c < 3; ++c)   // R (src/sim/simulation.cpp:151-158)
+                    tile[c * S + y * TC + l] =
+                        cadd(cadd(cadd(cscale(s.a0, u[b][c]), cscale(s.a1, up[b][c])), cscale(s.b0, nv[b][c])),
+                             cscale(s.b1, np[b][c]));
+                sy = cadd(sy, nv[b][1]);
+            }
+        }
+        tile[3 * S + g * TC + l] = sy;   // [16][TC], in P's tile until its first sweep
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+
+    // ---- chains ------------------------------------------------------------
+    // lane = 16 p + 2 cl + r: parity p, column cl of the block, part r (re, im)
+    const int p = lane >> 4, cl = (lane >> 1) & (TC - 1), r = lane & 1;
+    const int own = 2 * cl + r, oth = own ^ 1;
+    const int col = col0 + cl;
+    const bool live = col < ncol;
+    const int ccol = live ? col : ncol - 1;
+    const double ax = t.wavx[ccol % nkx], az = t.wavz[ccol / nkx];
+    const double sx = r ? ax : -ax, sz = r ? az : -az;
+    const bool zero_col = col == d.zc;
+    double *T = reinterpret_cast<double *>(tile);
+    const double *ad = s_ad + cl * AS;
+    bool pivot_fail = false;
+    // warps 1-3 hold the velocity pivots in registers while warp 0 solves the pressure
+    constexpr int kHoldCols = (TC + 2) / 3, kHoldRows = 8;   // NYS + 1 <= 256
+    double hold[kHoldCols][kHoldRows];
+    // warp 0's lanes fetch their column's influence data before the chains run:
+    // lane p uses sigma_0's entry p, and v of the first response at y = ny - p
+    const int coln = min(ccol / nkx, 2 * d.NZS - ccol / nkx) * nkx + ccol % nkx;   // the kz <= 0 column
+    double i00 = 0.0, i01 = 0.0, i10 = 0.0, i11 = 0.0, sg = 1.0, pn = 0.0, vn = 0.0, tail = 0.0;
+    if (w == 0) {
+        const double *sum = T + 6 * S;
+        double lower, upper;
+        // sums of N_y over this parity's rows, then over both
+        double mine = 0.0;
+#pragma unroll
+        for (int q = 0; q < kRowGroups / 2; ++q) mine += sum[(2 * q + p) * (2 * TC) + own];
+        const double other = __shfl_xor_sync(kFull, mine, 16);
+        const double even = p ? other : mine, odd = p ? mine : other;
+        if (s.bc_p) {
+            lower = reinterpret_cast<const double *>(s.bc_p + ccol)[r];
+            upper = reinterpret_cast<const double *>(s.bc_p + ncol + ccol)[r];
+        } else {
+            // pressure wall data (src/solver/eqsolve_pv.cpp:322-337) and its
+            // combination b0 B + b1 B_prev (src/sim/simulation.cpp:146-150)
+            const double bt = reinterpret_cast<const double *>(s.bw + ccol)[r] + (even + odd);
+            const double bb = reinterpret_cast<const double *>(s.bw + ncol + ccol)[r] + (odd - even);
+            lower = s.b0 * bt + s.b1 * reinterpret_cast<const double *>(s.B_prev + ccol)[r];
+            upper = s.b0 * bb + s.b1 * reinterpret_cast<const double *>(s.B_prev + ncol + ccol)[r];
+            if (live) reinterpret_cast<double *>(s.B_new + p * ncol + col)[r] = p ? bb : bt;
+        }
+        tail = T[(2 * S) + (ny - p) * (2 * TC) + own];   // R_1 at ny, ny - 1
+        {
+            const long long o_n = ((long long)(coln / nkx) * ncy + ny) * nkx + coln % nkx;
+            i00 = st.inf_div[coln].x;
+            i01 = st.inf_div[ncol + coln].x;
+            i10 = st.inf_div[2 * ncol + coln].x;
+            i11 = st.inf_div[3 * ncol + coln].x;
+            sg = st.sigma0[p * ncol + coln].x;
+            pn = st.p_inf[o_n];
+            vn = st.v_inf[d.Ns + o_n - p * nkx];
+        }
+        __syncwarp();   // the sums were read by every lane before P's sweep overwrites them
+        DivergenceRhs rhs{T + oth, T + 2 * S + own, T + 4 * S + oth, sx, sz, ny};
+        pivot_fail |= !tau_chain(ny, p, A.p_a, A.p_b, pp.G_pre == 0.0 && A.p_a == 0.0 && zero_col, lower, upper,
+                                 st.wn_p[ccol], s_w, t.WD, ad, T + 6 * S + own, rhs, [](double, double) {});
+    } else {
+#pragma unroll
+        for (int i = 0; i < kHoldCols; ++i) {
+            const int q = w - 1 + 3 * i;
+            const double *src = st.ad_v + pivot_base(min(q, TC - 1));
+#pragma unroll
+            for (int k = 0; k < kHoldRows; ++k) {
+                const int y = lane + 32 * k;
+                if (q < TC && y < ncy) hold[i][k] = src[y];
+            }
         }
     }
     __syncthreads();
-
-    if (col < ncol) {
-        const int kzi = col / nkx, kx = col - kzi * nkx;
-        const double ax = t.wavx[kx], az = t.wavz[kzi];
-        const bool zero_col = col == d.zc;
-        const long long cm = (long long)col * ncy;   // column-major base
-        bool pivot_fail = false;
-        double2 pv[E], v0[E], v1[E], v2[E], dy[E];
+    if (w > 0) {
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const int y = ycoef<E>(e);
-            if (y <= ny) {
-                const int sl = tile_slot<E>(y, w);
-                v0[e] = tile[sl];
-                v1[e] = tile[S + sl];
-                v2[e] = tile[2 * S + sl];
-                dy[e] = tile[3 * S + sl];
-            } else {
-                v0[e] = v1[e] = v2[e] = dy[e] = mk(0.0, 0.0);
+        for (int i = 0; i < kHoldCols; ++i) {
+            const int q = w - 1 + 3 * i;
+#pragma unroll
+            for (int k = 0; k < kHoldRows; ++k) {
+                const int y = lane + 32 * k;
+                if (q < TC && y < ncy) s_ad[q * AS + y] = hold[i][k];
             }
         }
-        double2 lower, upper;
-        if (s.bc_p) {
-            lower = s.bc_p[col];
-            upper = s.bc_p[ncol + col];
+    }
+    __syncthreads();
+    const double wv = st.wn_v[ccol];
+    if (w < 3) {
+        const double lower = reinterpret_cast<const double *>(s.bc_v + (2 * w) * ncol + ccol)[r];
+        const double upper = reinterpret_cast<const double *>(s.bc_v + (2 * w + 1) * ncol + ccol)[r];
+        const double a = w == 0 ? pp.a_V[0] : w == 1 ? pp.a_V[1] : pp.a_V[2];
+        const double b = w == 0 ? pp.b_V[0] : w == 1 ? pp.b_V[1] : pp.b_V[2];
+        const bool nrm = g_v == 0.0 && a == 0.0 && zero_col;
+        double *f = T + w * 2 * S + own;
+        double sum = 0.0;   // wall sums of this chain (src/solver/eqsolve_pv.cpp:397-406)
+        if (w == 1) {
+            VelocityRhs<1> rhs{T + 6 * S + own, f, 0.0, pp.Re, ny};
+            pivot_fail |= !tau_chain(ny, p, a, b, nrm, lower, upper, wv, s_w, t.WD, ad, f, rhs,
+                                     [&](double yd, double z) { sum += (yd * yd) * z; });
         } else {
-            // pressure wall data (src/solver/eqsolve_pv.cpp:322-337)
-            double2 st_ = mk(0, 0), sb_ = mk(0, 0);
-#pragma unroll
-            for (int e = 0; e < E; ++e) {
-                st_ = cadd(st_, dy[e]);
-                sb_ = p ? cadd(sb_, dy[e]) : csub(sb_, dy[e]);
-            }
-            st_ = sum_warp(st_);
-            sb_ = sum_warp(sb_);
-            const double2 bt = cadd(s.bw[col], st_);
-            const double2 bb = cadd(s.bw[ncol + col], sb_);
-            if (L == 0) {
-                s.B_new[col] = bt;
-                s.B_new[ncol + col] = bb;
-            }
-            // combined wall data b0 B + b1 B_prev (src/sim/simulation.cpp:146-150)
-            lower = cadd(cscale(s.b0, bt), cscale(s.b1, s.B_prev[col]));
-            upper = cadd(cscale(s.b0, bb), cscale(s.b1, s.B_prev[ncol + col]));
+            VelocityRhs<0> rhs{T + 6 * S + oth, f, w == 0 ? sx : sz, pp.Re, ny};
+            pivot_fail |= !tau_chain(ny, p, a, b, nrm, lower, upper, wv, s_w, t.WD, ad, f, rhs,
+                                     [&](double, double z) { sum += z; });
         }
-        // divergence of R (src/solver/eqsolve_pv.cpp:340-357)
-        deriv_warp<E>(ny, v1, dy);
-#pragma unroll
-        for (int e = 0; e < E; ++e)
-            if (ycoef<E>(e) <= ny) dy[e] = cadd(cadd(fderiv(ax, v0[e]), dy[e]), fderiv(az, v2[e]));
-        // pressure
-        double ad[E];
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const int y = ycoef<E>(e);
-            ad[e] = y <= ny ? st.ad_p[cm + y] : 0.0;
+        s_wall[w][p][own] = sum;
+    }
+    if (pivot_fail && live) atomicOr(s.err, ERR_PIVOT);
+    __syncthreads();
+
+    // ---- influence and sigma coefficients (src/solver/eqsolve_pv.cpp:397-429) ----
+    // The influence divergences and sigma_0 are real (real wall data, fields real
+    // or imaginary): part r of a column's coefficients needs only scalars.  Lane
+    // 16 q + 2 cl + r also divides by sigma_0's entry q.
+    if (w == 0 && live) {
+        // sums over parity q of i kx u + i kz w (this part) and of y^2 v
+        const double te = sx * s_wall[0][0][oth] + sz * s_wall[2][0][oth], ne = s_wall[1][0][own];
+        const double to = sx * s_wall[0][1][oth] + sz * s_wall[2][1][oth], no = s_wall[1][1][own];
+        const double div0 = (te + ne) + (to + no), div1 = (te - ne) + (no - to);
+        const double c0 = div1 * i10 - div0 * i11, c1 = div0 * i01 - div1 * i00;
+        const double cs = c0 + c1, cdf = c0 - c1;
+        const bool ev = (ny & 1) == 0;   // parity of ny
+        const double vt = T[2 * S + (ny - p) * (2 * TC) + own] + vn * (ev == (p == 0) ? cdf : cs);
+        double num;
+        if (p == 0) {
+            num = -wv * vt - pp.Re * tail;
+        } else {
+            const double ptop = T[6 * S + ny * (2 * TC) + own] + pn * (ev ? cs : cdf);
+            num = -wv * vt + pp.Re * (2.0 * ny * ptop - tail);
         }
-        pivot_fail |= !tau_warp<E>(ny, pp.G_pre, A.p_a, A.p_b, zero_col, lower, upper, st.wn_p[col], dy, pv,
-                                   ad, t.WL, t.WD, t.WR);
-        const double2 tail0 = elem<E>(v1, ny), tail1 = elem<E>(v1, ny - 1);
-        // velocity: Re (grad P - R) (src/solver/eqsolve_pv.cpp:359-395)
-        deriv_warp<E>(ny, pv, dy);
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const int y = ycoef<E>(e);
-            ad[e] = y <= ny ? st.ad_v[cm + y] : 0.0;
+        reinterpret_cast<double *>(s_sg[p])[own] = num / sg;
+        if (p == 0) {
+            reinterpret_cast<double *>(s_cs)[own] = cs;
+            reinterpret_cast<double *>(s_cd)[own] = cdf;
         }
-        const double wv = st.wn_v[col];
-        auto velocity = [&](int c, double2(&vc)[E]) {
-            double2 f[E];
-#pragma unroll
-            for (int e = 0; e < E; ++e) {
-                const double2 grad = (c == 0) ? fderiv(ax, pv[e]) : (c == 1) ? dy[e] : fderiv(az, pv[e]);
-                f[e] = ycoef<E>(e) <= ny ? cscale(pp.Re, csub(grad, vc[e])) : mk(0.0, 0.0);
-            }
-            const double2 blo = s.bc_v[(2 * c) * ncol + col], bup = s.bc_v[(2 * c + 1) * ncol + col];
-            pivot_fail |= !tau_warp<E>(ny, g_v, pp.a_V[c], pp.b_V[c], zero_col, blo, bup, wv, f, vc, ad,
-                                       t.WL, t.WD, t.WR);
-        };
-        velocity(0, v0);
-        velocity(1, v1);
-        velocity(2, v2);
-        // wall divergence by endpoint sums (src/solver/eqsolve_pv.cpp:397-406)
-        double2 div0 = mk(0, 0), div1 = mk(0, 0);
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const int y = ycoef<E>(e);
-            const double2 tang = cadd(fderiv(ax, v0[e]), fderiv(az, v2[e]));
-            const double2 nrm = cscale((double)(y * y), v1[e]);
-            div0 = cadd(div0, cadd(tang, nrm));
-            div1 = p ? cadd(div1, cadd(mk(-tang.x, -tang.y), nrm)) : cadd(div1, csub(tang, nrm));
-        }
-        div0 = sum_warp(div0);
-        div1 = sum_warp(div1);
-        // influence and sigma coefficients (src/solver/eqsolve_pv.cpp:408-429)
-        const double2 i00 = st.inf_div[col], i01 = st.inf_div[ncol + col];
-        const double2 i10 = st.inf_div[2 * ncol + col], i11 = st.inf_div[3 * ncol + col];
-        const double2 c0 = csub(cmul(div1, i10), cmul(div0, i11));
-        const double2 c1 = csub(cmul(div0, i01), cmul(div1, i00));
-        const long long o_n = ((long long)kzi * ncy + ny) * nkx + kx, o_n1 = o_n - nkx;
-        const double2 ptop = cadd(elem<E>(pv, ny), cadd(inf_mul(c0, st.p_inf[o_n], false),
-                                                        inf_mul(c1, st.p_inf[d.Ns + o_n], false)));
-        const double2 vt0 = cadd(elem<E>(v1, ny), cadd(inf_mul(c0, st.v_inf[d.Ns + o_n], false),
-                                                       inf_mul(c1, st.v_inf[4 * d.Ns + o_n], false)));
-        const double2 vt1 = cadd(elem<E>(v1, ny - 1), cadd(inf_mul(c0, st.v_inf[d.Ns + o_n1], false),
-                                                           inf_mul(c1, st.v_inf[4 * d.Ns + o_n1], false)));
-        const double2 n0 = csub(cscale(-wv, vt0), cscale(pp.Re, tail0));
-        const double2 n1 = cadd(cscale(-wv, vt1), cscale(pp.Re, csub(cscale(2.0 * ny, ptop), tail1)));
-        if (L == 0) {
-            s_c0[w] = c0;
-            s_c1[w] = c1;
-            s_sg[0][w] = cdiv(n0, st.sigma0[col]);
-            s_sg[1][w] = cdiv(n1, st.sigma0[ncol + col]);
-        }
-        // uncorrected solution into the tile (each warp rewrites only its own column's slots)
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const int y = ycoef<E>(e);
-            if (y > ny) continue;
-            const int sl = tile_slot<E>(y, w);
-            tile[sl] = pv[e];
-            tile[S + sl] = v0[e];
-            tile[2 * S + sl] = v1[e];
-            tile[3 * S + sl] = v2[e];
-        }
-        if (__any_sync(kFull, pivot_fail) && L == 0) atomicOr(s.err, ERR_PIVOT);
     }
     __syncthreads();
 
     // ---- influence and sigma corrections, coalesced over the block --------
-    // odd-y coefficients take sigma_0 for p, u, w and sigma_1 for v; even-y the reverse
+    // rows g, g + 16, ... all have the parity of g.  Odd-y coefficients take
+    // sigma_0 for p, u, w and sigma_1 for v, even-y the reverse; the second
+    // response's sign makes c0 + c1 the even p, u, w and odd v coefficient.
     const int zc = d.zc;   // the (kz, kx) = (0, 0) column (-1: not on this rank)
     const bool fix_zero = !s.solve_only && zc >= col0 && zc < col0 + TC;
     bool bad = false;
-    for (int i = tid; i < S; i += kThreads) {
-        const int y = i / TC, l = i - (i / TC) * TC;
-        const int c2 = col0 + l;
-        if (c2 >= ncol) continue;
-        const int kzi = c2 / nkx, kx = c2 - (c2 / nkx) * nkx;
-        const long long off = ((long long)kzi * ncy + y) * nkx + kx;
-        const int sl = tile_slot<E>(y, l);
-        const double2 c0 = s_c0[l], c1 = s_c1[l];
-        const double2 sq = s_sg[(y + 1) & 1][l], sv = s_sg[y & 1][l];
-        double2 pr = cadd(tile[sl], cadd(inf_mul(c0, st.p_inf[off], false), inf_mul(c1, st.p_inf[d.Ns + off], false)));
-        pr = cadd(pr, inf_mul(sq, st.p_b[off], false));
-        double2 v[3];
+    if (ok) {
+        const bool odd = g & 1;
+        const double2 cq = odd ? s_cd[l] : s_cs[l], cv = odd ? s_cs[l] : s_cd[l];
+        const double2 sq = s_sg[odd ? 0 : 1][l], sv = s_sg[odd ? 1 : 0][l];
+        const double axl = t.wavx[kx], azl = t.wavz[kzi];
+        const bool same_uw = pp.a_V[0] == pp.a_V[2] && pp.b_V[0] == pp.b_V[2];
+        // q = the stored field that gives both u and w: u (w = az/ax u) where kx > 0, w where kx = 0
+        const double sgn = kzi > d.NZS ? -1.0 : 1.0;   // w of the kz <= 0 column, negated
+        const double fu = axl != 0.0 ? 1.0 : 0.0;
+        const double fw = same_uw && axl != 0.0 ? azl / axl : sgn;
+        const long long comp = axl != 0.0 ? 0 : 2 * d.Ns;
+        const long long in0 = (long long)kzn * ncy * nkx + kx, out0 = (long long)kzi * ncy * nkx + kx;
+        constexpr int kBatch = 4;
+        for (int y0 = g; y0 < ncy; y0 += kBatch * kRowGroups) {
+            double pi[kBatch], qi[kBatch], vi[kBatch], wi[kBatch], pb[kBatch], qb[kBatch], vb[kBatch], wb[kBatch];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            v[c] = cadd(tile[(1 + c) * S + sl], cadd(inf_mul(c0, st.v_inf[c * d.Ns + off], inf_imag(c)),
-                                                     inf_mul(c1, st.v_inf[(3 + c) * d.Ns + off], inf_imag(c))));
-            v[c] = cadd(v[c], inf_mul(c == 1 ? sv : sq, st.v_b[c * d.Ns + off], inf_imag(c)));
+            for (int k = 0; k < kBatch; ++k) {
+                const long long o = in0 + (long long)min(y0 + k * kRowGroups, ny) * nkx;
+                pi[k] = ld256(st.p_inf + o);
+                vi[k] = ld256(st.v_inf + d.Ns + o);
+                pb[k] = ld256(st.p_b + o);
+                vb[k] = ld256(st.v_b + d.Ns + o);
+                qi[k] = ld256(st.v_inf + comp + o);
+                qb[k] = ld256(st.v_b + comp + o);
+                wi[k] = qi[k];
+                wb[k] = qb[k];
+                if (!same_uw && comp == 0) {
+                    wi[k] = st.v_inf[2 * d.Ns + o];
+                    wb[k] = st.v_b[2 * d.Ns + o];
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k) {
+                const int y = y0 + k * kRowGroups;
+                if (y >= ncy) break;
+                const int sl = y * TC + l;
+                const double2 pr = cadd(cadd(tile[3 * S + sl], cscale(pi[k], cq)), cscale(pb[k], sq));
+                double2 v[3];
+                v[0] = cadd(cadd(tile[sl], fderiv(fu * qi[k], cq)), fderiv(fu * qb[k], sq));
+                v[1] = cadd(cadd(tile[S + sl], cscale(vi[k], cv)), cscale(vb[k], sv));
+                v[2] = cadd(cadd(tile[2 * S + sl], fderiv(fw * wi[k], cq)), fderiv(fw * wb[k], sq));
+                if (fix_zero && c2 == zc) {
+                    tile[3 * S + sl] = pr;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) tile[c * S + sl] = v[c];
+                    continue;
+                }
+                bad |= !(isfinite(pr.x) && isfinite(pr.y) && isfinite(v[0].x) && isfinite(v[0].y) &&
+                         isfinite(v[1].x) && isfinite(v[1].y) && isfinite(v[2].x) && isfinite(v[2].y));
+                const long long o = out0 + (long long)y * nkx;
+                A.p_out[o] = pr;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) A.v_out[c * d.Ns + o] = v[c];
+                if (s.om) {
+                    s.om[d.Ns + o] = csub(fderiv(azl, v[0]), fderiv(axl, v[2]));
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) tile[c * S + sl] = v[c];
+                }
+            }
         }
-        if (fix_zero && c2 == zc) {
-            tile[sl] = pr;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) tile[(1 + c) * S + sl] = v[c];
-            continue;
-        }
-        bad |= !(isfinite(pr.x) && isfinite(pr.y) && isfinite(v[0].x) && isfinite(v[0].y) && isfinite(v[1].x) &&
-                 isfinite(v[1].y) && isfinite(v[2].x) && isfinite(v[2].y));
-        A.p_out[off] = pr;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) A.v_out[c * d.Ns + off] = v[c];
     }
     if (fix_zero) {
         __syncthreads();
-        if (w == zc - col0) {
-            const int kzi = d.NZS;
-            double2 pz[E], u0[E], u1[E], u2[E];
-#pragma unroll
-            for (int e = 0; e < E; ++e) {
-                const int y = ycoef<E>(e);
-                const int sl = tile_slot<E>(y <= ny ? y : 0, w);
-                pz[e] = tile[sl];
-                u0[e] = tile[S + sl];
-                u2[e] = tile[3 * S + sl];
-            }
+        if (w == 0) {
+            const int lz = zc - col0;
             // correct_zero_mode (src/solver/timestepper.cpp:60-68)
             const double2 v1w = cscale(0.5, cadd(s.bc_v[2 * ncol + zc], s.bc_v[3 * ncol + zc]));
-#pragma unroll
-            for (int e = 0; e < E; ++e) u1[e] = ycoef<E>(e) == 0 ? v1w : mk(0.0, 0.0);
             // correct_flow (src/sim/simulation.cpp:111-140), single-rank branch
             const double *uu = st.unit;
             double dpdx, dpdz;
@@ -375,13 +545,9 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
                 dpdz = pp.gz;
             } else {
                 double qx = 0.0, qz = 0.0;
-#pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    const int y = ycoef<E>(e);
-                    if (p == 0 && y <= ny) {
-                        qx += u0[e].x / (double)(y * y - 1);
-                        qz += u2[e].x / (double)(y * y - 1);
-                    }
+                for (int y = 2 * lane; y <= ny; y += 64) {
+                    qx += tile[y * TC + lz].x / (double)(y * y - 1);
+                    qz += tile[2 * S + y * TC + lz].x / (double)(y * y - 1);
                 }
                 qx = -sum_warp(qx);
                 qz = -sum_warp(qz);
@@ -390,31 +556,111 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
                 dpdx = (pp.qxm - qx) / qxu;
                 dpdz = (pp.qzm - qz) / qzu;
             }
-            if (L == 0) {
+            if (lane == 0) {
                 s.dpdx[0] = dpdx;
                 s.dpdx[1] = dpdz;
                 if (pfail) atomicOr(s.err, ERR_PIVOT);
             }
-#pragma unroll
-            for (int e = 0; e < E; ++e) {
-                const int y = ycoef<E>(e);
-                if (y > ny) continue;
-                u0[e].x += dpdx * uu[y];
-                u2[e].x += dpdz * uu[ncy + y];
-                bad |= !(isfinite(pz[e].x) && isfinite(pz[e].y) && isfinite(u0[e].x) && isfinite(u0[e].y) &&
-                         isfinite(u1[e].x) && isfinite(u1[e].y) && isfinite(u2[e].x) && isfinite(u2[e].y));
-                const long long off = ((long long)kzi * ncy + y) * nkx;
-                A.p_out[off] = pz[e];
-                A.v_out[off] = u0[e];
-                A.v_out[d.Ns + off] = u1[e];
-                A.v_out[2 * d.Ns + off] = u2[e];
+            for (int y = lane; y <= ny; y += 32) {
+                const double2 pz = tile[3 * S + y * TC + lz];
+                double2 u0 = tile[y * TC + lz], u2 = tile[2 * S + y * TC + lz];
+                const double2 u1 = y == 0 ? v1w : mk(0.0, 0.0);
+                u0.x += dpdx * uu[y];
+                u2.x += dpdz * uu[ncy + y];
+                bad |= !(isfinite(pz.x) && isfinite(pz.y) && isfinite(u0.x) && isfinite(u0.y) && isfinite(u1.x) &&
+                         isfinite(u1.y) && isfinite(u2.x) && isfinite(u2.y));
+                const long long off = ((long long)d.NZS * ncy + y) * nkx + (zc - d.NZS * nkx);
+                A.p_out[off] = pz;
+                A.v_out[off] = u0;
+                A.v_out[d.Ns + off] = u1;
+                A.v_out[2 * d.Ns + off] = u2;
+                if (s.om) {
+                    s.om[d.Ns + off] = mk(0.0, 0.0);
+                    tile[y * TC + lz] = u0;
+                    tile[S + y * TC + lz] = u1;
+                    tile[2 * S + y * TC + lz] = u2;
+                }
             }
         }
     }
-    if (__any_sync(kFull, bad) && L == 0) atomicOr(s.err, ERR_NONFINITE);
+    if (__any_sync(kFull, bad) && lane == 0) atomicOr(s.err, ERR_NONFINITE);
+    if (!s.om) return;
+
+    // ---- curl of the new velocity (src/solver/vector_ops.cpp:112-151), for the
+    // next step: om_x = dw/dy - i kz v, om_z = i kx v - du/dy (om_y is written
+    // above), and its pressure-wall sums.  Warps 0 and 1 differentiate u and w in
+    // place, warp 2 sums v: from the tile, this saves a kernel of its own that
+    // read the velocity back.
+    __syncthreads();
+    if (w < 3) {
+        double *f = T + (w == 0 ? 0 : w == 1 ? 4 * S : 2 * S) + own;
+        double sum = 0.0;
+        if (w < 2) {
+            // d_y = sum of 2 j f_j over j = y + 1, y + 3, ..., halved at y = 0, left
+            // in row y + 1, whose operand its thread has just read (d_NYS = 0)
+            double acc = 0.0;
+            int q = ((ny & 1) == p) ? ny - 1 : ny;   // rows of the other parity, descending
+            double qd = 2.0 * (double)q;
+            for (; q - 2 * (kRows - 1) >= 2; q -= 2 * kRows) {
+                double v[kRows];
+#pragma unroll
+                for (int i = 0; i < kRows; ++i) v[i] = (qd - (double)(4 * i)) * f[(q - 2 * i) * (2 * TC)];
+                qd -= (double)(4 * kRows);
+#pragma unroll
+                for (int i = 0; i < kRows; ++i) {
+                    acc += v[i];
+                    f[(q - 2 * i) * (2 * TC)] = acc;
+                    sum += acc;
+                }
+            }
+            for (; q >= 1; q -= 2, qd -= 4.0) {
+                acc += qd * f[q * (2 * TC)];
+                const double dv = q == 1 ? 0.5 * acc : acc;
+                f[q * (2 * TC)] = dv;
+                sum += dv;
+            }
+        } else {
+            for (int y = p; y <= ny; y += 2) sum += f[y * (2 * TC)];
+        }
+        s_wall[w][p][own] = sum;
+    }
+    __syncthreads();
+    if (ok) {
+        const double axl = t.wavx[kx], azl = t.wavz[kzi];
+        const long long out0 = (long long)kzi * ncy * nkx + kx;
+#pragma unroll 4
+        for (int y = g; y < ncy; y += kRowGroups) {
+            const int sl = y * TC + l;
+            const long long o = out0 + (long long)y * nkx;
+            const double2 v = tile[S + sl];
+            const double2 du = y < ny ? tile[sl + TC] : mk(0.0, 0.0), dw = y < ny ? tile[2 * S + sl + TC] : mk(0.0, 0.0);
+            s.om[o] = csub(dw, fderiv(azl, v));
+            s.om[2 * d.Ns + o] = csub(fderiv(axl, v), du);
+        }
+        if (tid < TC) {
+            // sums over y of i kx/Re om_z - i kz/Re om_x, signs (+1, (-1)^(y+1))
+            // (src/solver/timestepper.cpp:26-43)
+            double2 part[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const double2 du = mk(s_wall[0][q][2 * l], s_wall[0][q][2 * l + 1]);
+                const double2 dw = mk(s_wall[1][q][2 * l], s_wall[1][q][2 * l + 1]);
+                const double2 sv = mk(s_wall[2][q][2 * l], s_wall[2][q][2 * l + 1]);
+                part[q] = csub(fderiv(axl / pp.Re, csub(fderiv(axl, sv), du)),
+                               fderiv(azl / pp.Re, csub(dw, fderiv(azl, sv))));
+            }
+            s.bw_out[c2] = cadd(part[0], part[1]);
+            s.bw_out[ncol + c2] = csub(part[1], part[0]);
+        }
+    }
 }
 
-size_t solve_smem(const Dims &d) { return sizeof(double2) * 4 * (size_t)d.ncy * TC; }
+// the four tiles (P's holds the [16][TC] sums of N_y first, also where NYS + 1 < 16),
+// the row weights and the pivots
+size_t solve_smem(const Dims &d) {
+    const size_t tiles = 3 * (size_t)d.ncy * TC + (size_t)(d.ncy > kRowGroups ? d.ncy : kRowGroups) * TC;
+    return sizeof(double2) * (tiles + d.ncy) + sizeof(double) * TC * (size_t)pivot_stride(d.ncy);
+}
 
 __global__ void k_pressure_bc(Dims d, const double2 *N, const double2 *bw, double2 *B) {
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
@@ -431,17 +677,6 @@ __global__ void k_pressure_bc(Dims d, const double2 *N, const double2 *bw, doubl
     B[d.ncol + col] = cadd(bw[d.ncol + col], sb_);
 }
 
-template <int E>
-cudaError_t configure_e(const Dims &d) {
-    return raise_smem(k_solve<E>, (int)solve_smem(d));
-}
-
-template <int E>
-void step_e(const Dims &d, const Tables &t, const PhysParams &pp, double g_v, const SolverState &st,
-            const SolveArgs &A, cudaStream_t s) {
-    const int blocks = (d.ncol + TC - 1) / TC;
-    k_solve<E><<<blocks, kThreads, solve_smem(d), s>>>(d, t, pp, g_v, st, A);
-}
 }  // namespace
 
 void launch_pressure_bc(const Dims &d, const double2 *N, const double2 *bw, double2 *B,
@@ -452,13 +687,8 @@ void launch_pressure_bc(const Dims &d, const double2 *N, const double2 *bw, doub
 cudaError_t configure_solver_kernels(const Dims &d) {
     cudaError_t e = configure_setup_kernels(d);
     if (e != cudaSuccess) return e;
-    switch (lane_elems(d)) {
-    case 1: return configure_e<1>(d);
-    case 2: return configure_e<2>(d);
-    case 4: return configure_e<4>(d);
-    case 8: return configure_e<8>(d);
-    default: return cudaErrorInvalidValue;   // more than 256 Chebyshev coefficients
-    }
+    if (lane_elems(d) == 0) return cudaErrorInvalidValue;   // more than 256 Chebyshev coefficients
+    return raise_smem(k_solve, solve_smem(d));
 }
 
 void launch_step_solve(const Dims &d, const Tables &t, const PhysParams &pp, double g_v,
@@ -469,13 +699,8 @@ void launch_step_solve(const Dims &d, const Tables &t, const PhysParams &pp, dou
     A.p_out = a.p_out;
     A.v_out = a.u_out;
     A.step = a;
-    switch (lane_elems(d)) {
-    case 1: step_e<1>(d, t, pp, g_v, st, A, s); break;
-    case 2: step_e<2>(d, t, pp, g_v, st, A, s); break;
-    case 4: step_e<4>(d, t, pp, g_v, st, A, s); break;
-    case 8: step_e<8>(d, t, pp, g_v, st, A, s); break;
-    default: break;
-    }
+    const int blocks = (d.ncol + TC - 1) / TC;
+    k_solve<<<blocks, kThreads, solve_smem(d), s>>>(d, t, pp, g_v, st, A);
 }
 
 }  // namespace cdns

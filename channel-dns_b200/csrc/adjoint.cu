@@ -203,7 +203,7 @@ k_solve_adj(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, AdjArgs
         const int c2 = col0 + l;
         if (c2 >= ncol) continue;
         const int kzi = c2 / nkx, kx = c2 - (c2 / nkx) * nkx;
-        const long long off = ((long long)kzi * ncy + y) * nkx + kx;
+        const long long off = spectral_base(d, kzi, kx) + (long long)y * d.sy;
         const int sl = tile_slot<E>(y, l);
         const double2 lp = A.lp ? A.lp[off] : mk(0.0, 0.0);
         double2 lv[3];
@@ -275,7 +275,7 @@ k_solve_adj(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, AdjArgs
         const double2 lvt0 = cscale(-wv, ln0), lvt1 = cscale(-wv, ln1);
         const double2 ltail0 = cscale(-pp.Re, ln0), ltail1 = cscale(-pp.Re, ln1);
         const double2 lptop = cscale(pp.Re * 2.0 * ny, ln1);
-        const long long o_n = ((long long)kzi * ncy + ny) * nkx + kx, o_n1 = o_n - nkx;
+        const long long o_n = spectral_base(d, kzi, kx) + (long long)ny * d.sy, o_n1 = o_n - d.sy;
         lc0 = cadd(lc0, cadd(cmulc_inf(st.p_inf[o_n], false, lptop),
                              cadd(cmulc_inf(st.v_inf[Ns + o_n], false, lvt0), cmulc_inf(st.v_inf[Ns + o_n1], false, lvt1))));
         lc1 = cadd(lc1, cadd(cmulc_inf(st.p_inf[Ns + o_n], false, lptop),
@@ -393,7 +393,7 @@ k_solve_adj(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, AdjArgs
         const int c2 = col0 + l;
         if (c2 >= ncol) continue;
         const int kzi = c2 / nkx, kx = c2 - (c2 / nkx) * nkx;
-        const long long off = ((long long)kzi * ncy + y) * nkx + kx;
+        const long long off = spectral_base(d, kzi, kx) + (long long)y * d.sy;
         const int sl = tile_slot<E>(y, l);
         if (!A.acc) {
 #pragma unroll
@@ -517,7 +517,7 @@ k_curl_adj(Dims d, Tables t, const double2 *__restrict__ lS, const double2 *__re
         const int c2 = col0 + l;
         if (c2 >= ncol) continue;
         const int kzi = c2 / nkx, kx = c2 - (c2 / nkx) * nkx;
-        const long long off = ((long long)kzi * ncy + y) * nkx + kx;
+        const long long off = spectral_base(d, kzi, kx) + (long long)y * d.sy;
         const int sl = tile_slot<E>(y, l);
 #pragma unroll
         for (int c = 0; c < 3; ++c) tile[c * S + sl] = lS[(3 + c) * d.Ns + off];
@@ -562,7 +562,7 @@ k_curl_adj(Dims d, Tables t, const double2 *__restrict__ lS, const double2 *__re
         const int c2 = col0 + l;
         if (c2 >= ncol) continue;
         const int kzi = c2 / nkx, kx = c2 - (c2 / nkx) * nkx;
-        const long long off = ((long long)kzi * ncy + y) * nkx + kx;
+        const long long off = spectral_base(d, kzi, kx) + (long long)y * d.sy;
         const int sl = tile_slot<E>(y, l);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -577,13 +577,14 @@ size_t curl_adj_smem(const Dims &d) { return sizeof(double2) * 3 * (size_t)d.ncy
 // lN_y += the transposed wall sums of lB (standalone nonlinear adjoint).
 __global__ void k_pressure_bc_adj(Dims d, const double2 *__restrict__ lB, double2 *__restrict__ lN) {
     const long long ncol = d.ncol;
-    for (long long off = blockIdx.x * (long long)blockDim.x + threadIdx.x; off < d.Ns;
-         off += (long long)gridDim.x * blockDim.x) {
-        const int kx = (int)(off % d.nkx);
-        const long long q = off / d.nkx;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < d.Nl;
+         i += (long long)gridDim.x * blockDim.x) {
+        const int kx = (int)(i % d.nkx);
+        const long long q = i / d.nkx;
         const int y = (int)(q % d.ncy), kzi = (int)(q / d.ncy);
         const long long col = (long long)kzi * d.nkx + kx;
-        const double2 bt = lB[col], bb = lB[ncol + col];
+        const long long off = spectral_base(d, kzi, kx) + (long long)y * d.sy;
+        const double2 bt = lB[col], bb = lB[d.ncol + col];
         lN[d.Ns + off] = cadd(lN[d.Ns + off], (y & 1) ? cadd(bt, bb) : csub(bt, bb));
     }
 }
@@ -594,7 +595,7 @@ __global__ void k_wall_shear(Dims d, const double2 *__restrict__ u, double re, d
     const int L = threadIdx.x;
     double acc = 0.0;
     for (int y = 2 * L; y <= d.NYS; y += 64) {
-        const long long off = ((long long)d.NZS * d.ncy + y) * d.nkx;
+        const long long off = spectral_base(d, d.NZS, 0) + (long long)y * d.sy;
         acc += (double)(y * y) * u[off].x;
     }
     acc = sum_warp(acc);

@@ -304,16 +304,16 @@ int cdns_adjoint_run(cdns_ctx *c, int nsteps, int kck, int objective, const doub
         if (shear) launch_wall_shear(d, c->U[c->cur], c->pp.Re, w->jbuf + it - 1, s);
     }
     CK(cudaGetLastError());
-    const size_t n3 = 3 * (size_t)d.Ns, nc = d.ncol;
+    const size_t n3 = 3 * (size_t)d.Ns, n3l = 3 * (size_t)d.Nl, nc = d.ncol;
     double Jp = 0.0;
     if (!shear) {
         // J = Re <w, u^nsteps>, in a fixed order on the host
-        std::vector<double> hu(2 * n3);
-        launch_interleave(c->U[c->cur], c->aux, d.Ns, 3, s);
+        std::vector<double> hu(2 * n3l);
+        launch_interleave(d, c->U[c->cur], c->aux, 3, s);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(hu.data(), c->aux, n3 * sizeof(double2), cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(hu.data(), c->aux, n3l * sizeof(double2), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        for (size_t i = 0; i < 2 * n3; ++i) Jp += weights[i] * hu[i];
+        for (size_t i = 0; i < 2 * n3l; ++i) Jp += weights[i] * hu[i];
     }
     if (grad) {
         if ((r = save_checkpoint(c, (size_t)nseg))) return r;
@@ -325,8 +325,8 @@ int cdns_adjoint_run(cdns_ctx *c, int nsteps, int kck, int objective, const doub
         CK(cudaMemsetAsync(w->lbcv, 0, 6 * nc * sizeof(double2), s));
         if (!shear) {
             // terminal seed: lu^nsteps = w
-            CK(cudaMemcpyAsync(c->aux2, weights, n3 * sizeof(double2), cudaMemcpyHostToDevice, s));
-            launch_deinterleave(c->aux2, w->lU[nsteps & 1], d.Ns, 3, s);
+            CK(cudaMemcpyAsync(c->aux2, weights, n3l * sizeof(double2), cudaMemcpyHostToDevice, s));
+            launch_deinterleave(d, c->aux2, w->lU[nsteps & 1], 3, s);
         }
         const double seed = shear ? -1.0 / ((double)nsteps * c->pp.Re) : 0.0;
         // ---- reverse sweep: the reverse steps of interval seg run on the
@@ -360,9 +360,9 @@ int cdns_adjoint_run(cdns_ctx *c, int nsteps, int kck, int objective, const doub
         CK(cudaEventRecord(w->ev_done, rs));
         CK(cudaStreamWaitEvent(s, w->ev_done, 0));
         if (grad_u) {
-            launch_interleave(w->lU[0], c->aux, d.Ns, 3, s);
+            launch_interleave(d, w->lU[0], c->aux, 3, s);
             CK(cudaGetLastError());
-            CK(cudaMemcpyAsync(grad_u, c->aux, n3 * sizeof(double2), cudaMemcpyDeviceToHost, s));
+            CK(cudaMemcpyAsync(grad_u, c->aux, n3l * sizeof(double2), cudaMemcpyDeviceToHost, s));
         }
         std::vector<double2> hb(grad_bc ? 6 * nc : 0);
         if (grad_bc) CK(cudaMemcpyAsync(hb.data(), w->lbcv, hb.size() * sizeof(double2), cudaMemcpyDeviceToHost, s));
@@ -391,15 +391,18 @@ int cdns_solve_adjoint(cdns_ctx *c, double g, const double *lp, const double *lv
     int r = do_setup(c, g);
     if (r || (r = ensure_work(c, 0, 0, 0))) return r;
     AdjointWork *w = c->adj;
-    const size_t Ns = (size_t)d.Ns, nc = d.ncol;
-    if (lp) CK(cudaMemcpyAsync(c->F, lp, Ns * sizeof(double2), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(c->aux2, lv, 3 * Ns * sizeof(double2), cudaMemcpyHostToDevice, s));
-    launch_deinterleave(c->aux2, c->aux, d.Ns, 3, s);
+    const size_t Nl = (size_t)d.Nl, nc = d.ncol;
+    if (lp) {
+        CK(cudaMemcpyAsync(c->H, lp, Nl * sizeof(double2), cudaMemcpyHostToDevice, s));
+        launch_deinterleave(d, c->H, c->F, 1, s);
+    }
+    CK(cudaMemcpyAsync(c->aux2, lv, 3 * Nl * sizeof(double2), cudaMemcpyHostToDevice, s));
+    launch_deinterleave(d, c->aux2, c->aux, 3, s);
     CK(cudaMemsetAsync(w->lbcv, 0, 6 * nc * sizeof(double2), s));
     launch_solve_adjoint(d, c->t, c->pp, g, c->st, lp ? c->F : nullptr, c->aux, w->lR, w->lBc, w->lbcv, 1, 0.0, s);
-    launch_interleave(w->lR, c->aux2, d.Ns, 3, s);
+    launch_interleave(d, w->lR, c->aux2, 3, s);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(lrhs, c->aux2, 3 * Ns * sizeof(double2), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(lrhs, c->aux2, 3 * Nl * sizeof(double2), cudaMemcpyDeviceToHost, s));
     std::vector<double2> hp(2 * nc), hv(6 * nc);
     CK(cudaMemcpyAsync(hp.data(), w->lBc, hp.size() * sizeof(double2), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(hv.data(), w->lbcv, hv.size() * sizeof(double2), cudaMemcpyDeviceToHost, s));
@@ -420,12 +423,12 @@ int cdns_nonlinear_adjoint(cdns_ctx *c, const double *velocity, const double *lN
     cudaStream_t s = c->stream;
     if ((r = ensure_work(c, 0, 1, 0))) return r;
     AdjointWork *w = c->adj;
-    const size_t Ns = (size_t)d.Ns, nc = d.ncol;
-    CK(cudaMemcpyAsync(c->aux2, velocity, 3 * Ns * sizeof(double2), cudaMemcpyHostToDevice, s));
-    launch_deinterleave(c->aux2, c->aux, d.Ns, 3, s);
+    const size_t Ns = (size_t)d.Ns, Nl = (size_t)d.Nl, nc = d.ncol;
+    CK(cudaMemcpyAsync(c->aux2, velocity, 3 * Nl * sizeof(double2), cudaMemcpyHostToDevice, s));
+    launch_deinterleave(d, c->aux2, c->aux, 3, s);
     enqueue_nonlinear(c, c->aux, w->lR, false, 0, w->gs);
-    CK(cudaMemcpyAsync(c->aux2, lN, 3 * Ns * sizeof(double2), cudaMemcpyHostToDevice, s));
-    launch_deinterleave(c->aux2, w->lN[0], d.Ns, 3, s);
+    CK(cudaMemcpyAsync(c->aux2, lN, 3 * Nl * sizeof(double2), cudaMemcpyHostToDevice, s));
+    launch_deinterleave(d, c->aux2, w->lN[0], 3, s);
     std::vector<double2> hb(2 * nc, make_double2(0.0, 0.0));
     if (lpbc) {
         const double2 *src = reinterpret_cast<const double2 *>(lpbc);
@@ -438,9 +441,9 @@ int cdns_nonlinear_adjoint(cdns_ctx *c, const double *velocity, const double *lN
     launch_pressure_bc_adjoint(d, w->lbw, w->lN[0], s);
     CK(cudaMemsetAsync(w->lU[0], 0, 3 * Ns * sizeof(double2), s));
     nonlinear_adjoint(c, w->gs, w->lN[0], w->lbw, w->lU[0], s);
-    launch_interleave(w->lU[0], c->aux2, d.Ns, 3, s);
+    launch_interleave(d, w->lU[0], c->aux2, 3, s);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(lu, c->aux2, 3 * Ns * sizeof(double2), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(lu, c->aux2, 3 * Nl * sizeof(double2), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     return CDNS_OK;
 }

@@ -320,7 +320,7 @@ k_ydct_any(Dims d, int N1, int N2, int TL, int R, const double2 *__restrict__ ro
         const double2 *S = nullptr;
         const CT *F = nullptr;
         if (!ANA) S = (f < A.nsplit ? A.spec0 + (long long)f * d.Ns : A.spec1 + (long long)(f - A.nsplit) * d.Ns) +
-                      (long long)kzi * ncy * nkx + kx;
+                      spectral_base(d, kzi, kx);
         else F = A.Fin + (long long)f * d.ny2 * d.fcol + (long long)kzi * nkx + kx;
         for (int n0 = r; n0 <= N / 2; n0 += kYPairs * R) {
             double2 xa[kYPairs], xb[kYPairs];
@@ -329,8 +329,8 @@ k_ydct_any(Dims d, int N1, int N2, int TL, int R, const double2 *__restrict__ ro
                 const int n = n0 + R * i, m = N - n;
                 const bool in = n <= N / 2 && lok;
                 if (!ANA) {
-                    xa[i] = (in && n < ncy) ? S[(long long)n * nkx] : mk(0.0, 0.0);
-                    xb[i] = (in && m < ncy) ? S[(long long)m * nkx] : mk(0.0, 0.0);
+                    xa[i] = (in && n < ncy) ? S[(long long)n * d.sy] : mk(0.0, 0.0);
+                    xb[i] = (in && m < ncy) ? S[(long long)m * d.sy] : mk(0.0, 0.0);
                 } else {
                     xa[i] = in ? cto<double2>(F[(long long)n * d.fcol]) : mk(0.0, 0.0);
                     xb[i] = in ? cto<double2>(F[(long long)m * d.fcol]) : mk(0.0, 0.0);
@@ -393,7 +393,7 @@ k_ydct_any(Dims d, int N1, int N2, int TL, int R, const double2 *__restrict__ ro
     CT *Fo = nullptr;
     double2 *So = nullptr;
     if (!ANA) Fo = A.Fout + (long long)f * d.ny2 * d.fcol + (long long)kzi * nkx + kx;
-    else So = A.S + (long long)f * d.Ns + (long long)kzi * ncy * nkx + kx;
+    else So = A.S + (long long)f * d.Ns + spectral_base(d, kzi, kx);
     const bool to_mean = !ANA && A.mean && kzi == d.NZS && kx == 0;
     auto out = [&](int j, double2 v) {
         if (!lok) return;
@@ -405,7 +405,7 @@ k_ydct_any(Dims d, int N1, int N2, int TL, int R, const double2 *__restrict__ ro
                 Fo[(long long)j * d.fcol] = cto<CT>(cscale(j == 0 || j == N ? A.outE : A.outI, v));
             }
         } else if (j < ncy) {
-            So[(long long)j * nkx] = cscale(j == 0 ? A.s0 : A.sk, v);
+            So[(long long)j * d.sy] = cscale(j == 0 ? A.s0 : A.sk, v);
         }
     };
     double2 part[kYChunk];

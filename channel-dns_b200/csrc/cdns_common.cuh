@@ -1,10 +1,14 @@
 // Shared device-side definitions for the channel-dns B200 step.
 //
-// Spectral fields live in HBM component-planar: component c of a vector field
-// is a contiguous complex<double> array [kz+NZS][y][kx] (the reference's
-// per-component order, src/core/array4d.hpp:62-67, with the component index
-// moved outermost).  The flattened column index col = kz_idx*nkx + kx numbers
-// the independent (kz, kx) Fourier modes.
+// Spectral fields live in HBM component-planar and tiled: the flattened column
+// index col = kz_idx*nkx + kx numbers the independent (kz, kx) Fourier modes, and
+// component c of a vector field is an array [col / 8][y][col mod 8] (Dims::Ns values
+// apart), so that the eight columns of a solve or curl block are one contiguous
+// run, aligned to 128-byte lines in every row.  (With the reference's order
+// [kz][y][kx], src/core/array4d.hpp:62-67, a block's rows are 128 bytes every
+// 16 nkx, at odd alignments: read at 2.7 TB/s on a B200, against 3.6 for aligned
+// rows and 6.2 for a linear array.)  Arrays that cross the C ABI are in the
+// reference's order; layout.cu converts.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -21,7 +25,11 @@ struct Dims {
     int fcol;            // row stride (columns) of the y-physical stage buffer F:
                          // ncol, rounded up to even for FP32 stages (16-byte rows)
     int nyh;             // NY2/2+1 (half of the y points, symmetric pairs)
-    long long Ns;        // nkz*ncy*nkx complex values per spectral component
+    long long Ns;        // complex values from one spectral component to the next
+    long long Nl;        // nkz*ncy*nkx, the values of a component in the reference's order
+    bool tiled;          // spectral arrays in the tiled layout (false: the reference's order)
+    int sy;              // distance of a column's coefficients y and y + 1: 8 (tiled), or nkx for
+                         // an array in the reference's order (planar_dims)
     int ztl;             // kx lines per block of the z transforms (0: the padding rule)
     int xrw;             // register-form x stage: (z, y) rows per block (2 or 4; 0: 4), 3 or 5:
                          // 4 or 2 rows with the forward phases split over lane pairs (even N1,
@@ -29,6 +37,30 @@ struct Dims {
     int kx0;             // global kx of local column kx = 0 (a pencil rank's kx block; else 0)
     int zc;              // local index of the (kz, kx) = (0, 0) column, -1 if not held here
 };
+
+constexpr int kTileCols = 8;   // columns of a spectral tile
+
+// Offset of coefficient y = 0 of the column (kz index kzi, kx) in a spectral
+// component; coefficient y is y * d.sy further.
+__host__ __device__ inline long long spectral_base(const Dims &d, int kzi, int kx) {
+    const int col = kzi * d.nkx + kx;
+    return d.tiled ? (long long)(col / kTileCols) * d.ncy * kTileCols + col % kTileCols
+                             : (long long)kzi * d.ncy * d.nkx + kx;
+}
+// Sizes and strides of the tiled layout / of spectral arrays in the reference's order.
+inline void set_tiled(Dims &d) {
+    d.Nl = (long long)d.nkz * d.ncy * d.nkx;
+    d.tiled = true;
+    d.sy = kTileCols;
+    d.Ns = (long long)((d.ncol + kTileCols - 1) / kTileCols) * kTileCols * d.ncy;
+}
+inline Dims planar_dims(Dims d) {
+    d.Nl = (long long)d.nkz * d.ncy * d.nkx;
+    d.tiled = false;
+    d.sy = d.nkx;
+    d.Ns = d.Nl;
+    return d;
+}
 
 // Read-only per-context tables in device memory.
 struct Tables {

@@ -107,7 +107,7 @@ void launch_x_adjoint(const Dims &d, const FftPlan &P, const double2 *roots, con
 struct SolverState {
     double *wn_p, *wn_v;        // [ncol]
     double *ad_p, *ad_v;        // [ncol][ncy] (column-major)
-    // Influence and B-problem fields, planar, each stored by its one nonzero
+    // Influence and B-problem fields, each stored by its one nonzero
     // part: the pressure and v are real, u and w purely imaginary (real wall
     // data and real operators; i kx, i kz enter only through the gradient), so
     // the other part is an exact zero and is not kept (inf_part).
@@ -139,7 +139,7 @@ struct PhysParams {
 };
 
 struct StepArgs {
-    const double2 *u, *u_prev, *N, *N_prev;   // planar 3-component spectral fields
+    const double2 *u, *u_prev, *N, *N_prev;   // 3-component spectral fields
     const double2 *bw;          // [2][ncol] vorticity part of the wall condition
     const double2 *B_prev;      // [2][ncol]
     double2 *B_new;             // [2][ncol]
@@ -196,7 +196,8 @@ void launch_wall_shear(const Dims &d, const double2 *u, double re, double *out, 
 int record_error(int code, const char *msg);
 
 // ---- layout.cu ----
-void launch_deinterleave(const double2 *src, double2 *dst, long long n, int nc, cudaStream_t s);
-void launch_interleave(const double2 *src, double2 *dst, long long n, int nc, cudaStream_t s);
+// nc components of the context's spectral arrays (nc = 1: a scalar field)
+void launch_deinterleave(const Dims &d, const double2 *src, double2 *dst, int nc, cudaStream_t s);
+void launch_interleave(const Dims &d, const double2 *src, double2 *dst, int nc, cudaStream_t s);
 
 }  // namespace cdns

@@ -113,7 +113,7 @@ k_curl(Dims d, Tables t, const double2 *__restrict__ u, double2 *__restrict__ om
             const int c2 = col0 + l;
             const bool ok = i < S && c2 < ncol;
             const int kzi = c2 / nkx, kx = c2 - (c2 / nkx) * nkx;
-            const long long off = ((long long)kzi * ncy + y) * nkx + kx;
+            const long long off = spectral_base(d, kzi, kx) + (long long)y * d.sy;
 #pragma unroll
             for (int c = 0; c < 3; ++c) v[b][c] = ok ? u[c * d.Ns + off] : mk(0.0, 0.0);
         }
@@ -177,7 +177,7 @@ k_curl(Dims d, Tables t, const double2 *__restrict__ u, double2 *__restrict__ om
         const int c2 = col0 + l;
         if (c2 >= ncol) continue;
         const int kzi = c2 / nkx, kx = c2 - (c2 / nkx) * nkx;
-        const long long off = ((long long)kzi * ncy + y) * nkx + kx;
+        const long long off = spectral_base(d, kzi, kx) + (long long)y * d.sy;
         const int sl = tile_slot<E>(y, l);
 #pragma unroll
         for (int c = 0; c < 3; ++c) om[c * d.Ns + off] = tile[c * S + sl];
@@ -242,7 +242,7 @@ k_ysynth(Dims d, const double *__restrict__ csyn, int jp, const double2 *__restr
                 const bool ok = k >= 0 && col < ncol;
                 const int kzi = ok ? col / d.nkx : 0, kx = ok ? col - kzi * d.nkx : 0;
                 cp_async16(xs + ((buf * 2 + (k & 1)) * KH + (r >> 1)) * kXS + l,
-                           X + ((long long)kzi * d.ncy + (ok ? k : 0)) * d.nkx + kx, ok ? 16 : 0);
+                           X + spectral_base(d, kzi, kx) + (long long)(ok ? k : 0) * d.sy, ok ? 16 : 0);
             } else {
                 const int c = u - nxu;
                 const int r = c / (jw / 2), h = c - r * (jw / 2);
@@ -329,7 +329,7 @@ k_ysynth(Dims d, const double *__restrict__ csyn, int jp, const double2 *__restr
 }
 
 // ---------------------------------------------------------------------------
-// Analysis: S[f][k][col] (spectral, planar) from F[f][j][col].  Grid (column
+// Analysis: S[f][k][col] (spectral) from F[f][j][col].  Grid (column
 // tiles of 32, fields); block (32, 2 G): warp (g, p) owns k = 2 m + p for
 // m = 16 g .. 16 g + 15, accumulated with 8x8x4 FP64 MMA over chunks of JC
 // points j; rows j and N - j are staged by cp.async and folded into
@@ -444,7 +444,7 @@ k_yanalysis(Dims d, const double *__restrict__ cana, int kh, const CI *__restric
             const int col = col0 + 4 * q + t;
             if (col >= ncol) continue;
             const int kzi = col / d.nkx, kx = col - kzi * d.nkx;
-            Sf[((long long)kzi * d.ncy + k) * d.nkx + kx] = cscale(k == 0 ? s0 : sn, mk(acc[mr][q][0], acc[mr][q][1]));
+            Sf[spectral_base(d, kzi, kx) + (long long)k * d.sy] = cscale(k == 0 ? s0 : sn, mk(acc[mr][q][0], acc[mr][q][1]));
         }
     }
 }
@@ -480,7 +480,7 @@ __global__ void k_mean_products(Dims d, const double *__restrict__ cana, int kh,
     acc = sum_warp(acc);
     if (lane == 0) {
         const double sc = k == 0 ? 1.0 / (2.0 * N) : 1.0 / (double)N;
-        double2 *s = S + (long long)c * d.Ns + ((long long)d.NZS * d.ncy + k) * d.nkx;   // kx = 0
+        double2 *s = S + (long long)c * d.Ns + spectral_base(d, d.NZS, 0) + (long long)k * d.sy;
         s->x += sc * acc;
     }
 }

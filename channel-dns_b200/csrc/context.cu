@@ -270,7 +270,7 @@ int create_context(const cdns_mesh_desc *m, const cdns_params *p, int precision,
     d.ncol = d.nkx * d.nkz;
     d.zc = d.kx0 == 0 ? d.NZS * d.nkx : -1;
     d.nyh = m->NY2 / 2 + 1;
-    d.Ns = (long long)d.nkz * d.ncy * d.nkx;
+    set_tiled(d);
     if (!plan_fft(d.NX2, c->px) || !plan_fft(d.NZ2, c->pz)) {
         delete c;
         return fail(CDNS_ERR_ARG, "NX2/NZ2 must factor into primes <= 13");
@@ -370,7 +370,8 @@ int create_context(const cdns_mesh_desc *m, const cdns_params *p, int precision,
     }
     // ---- state and workspaces ----
     const size_t Ns = (size_t)d.Ns, nc = d.ncol;
-    const size_t fbuf = 6 * (size_t)d.ny2 * nc;
+    // (F also takes the pressure of a standalone solve, a tiled component)
+    const size_t fbuf = std::max(6 * (size_t)d.ny2 * nc, Ns);
     const size_t gbuf = 6 * (size_t)d.ny2 * d.NZ2 * d.nkx;
     const size_t hbuf = 3 * (size_t)d.ny2 * d.NZ2 * d.nkx;
     if ((r = c->alloc(c->U[0], 3 * Ns)) || (r = c->alloc(c->U[1], 3 * Ns)) ||
@@ -445,7 +446,7 @@ int cdns_set_velocity_device(cdns_ctx *c, const double *v) {
     const Dims &d = c->d;
     c->cur = 0;
     c->om_current = false;
-    launch_deinterleave(reinterpret_cast<const double2 *>(v), c->U[0], d.Ns, 3, c->stream);
+    launch_deinterleave(d, reinterpret_cast<const double2 *>(v), c->U[0], 3, c->stream);
     CK(cudaMemsetAsync(c->U[1], 0, sizeof(double2) * 3 * d.Ns, c->stream));
     CK(cudaMemsetAsync(c->Nb[0], 0, sizeof(double2) * 3 * d.Ns, c->stream));
     CK(cudaMemsetAsync(c->Nb[1], 0, sizeof(double2) * 3 * d.Ns, c->stream));
@@ -459,7 +460,7 @@ int cdns_set_velocity_device(cdns_ctx *c, const double *v) {
 int cdns_set_velocity(cdns_ctx *c, const double *v) {
     if (!c || !v) return fail(CDNS_ERR_ARG, "null argument");
     DeviceGuard guard(c->device);
-    CK(cudaMemcpyAsync(c->aux, v, sizeof(double2) * 3 * c->d.Ns, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->aux, v, sizeof(double2) * 3 * c->d.Nl, cudaMemcpyHostToDevice, c->stream));
     int r = cdns_set_velocity_device(c, reinterpret_cast<const double *>(c->aux));
     if (r) return r;
     CK(cudaStreamSynchronize(c->stream));
@@ -471,10 +472,10 @@ int cdns_update_velocity(cdns_ctx *c, const double *v) {
     if (int r = require_whole(c)) return r;
     if (!c->have_velocity) return fail(CDNS_ERR_STATE, "cdns_update_velocity before cdns_set_velocity");
     DeviceGuard guard(c->device);
-    CK(cudaMemcpyAsync(c->aux, v, sizeof(double2) * 3 * c->d.Ns, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->aux, v, sizeof(double2) * 3 * c->d.Nl, cudaMemcpyHostToDevice, c->stream));
     // the current slot only: u_prev, N_prev and B_prev of the multistep history stay
     c->om_current = false;
-    launch_deinterleave(reinterpret_cast<const double2 *>(c->aux), c->U[c->cur], c->d.Ns, 3, c->stream);
+    launch_deinterleave(c->d, reinterpret_cast<const double2 *>(c->aux), c->U[c->cur], 3, c->stream);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->stream));
     return CDNS_OK;
@@ -484,7 +485,7 @@ int cdns_get_velocity_device(cdns_ctx *c, double *v) {
     if (!c || !v) return fail(CDNS_ERR_ARG, "null argument");
     if (!c->have_velocity) return fail(CDNS_ERR_STATE, "no velocity set");
     DeviceGuard guard(c->device);
-    launch_interleave(c->U[c->cur], reinterpret_cast<double2 *>(v), c->d.Ns, 3, c->stream);
+    launch_interleave(c->d, c->U[c->cur], reinterpret_cast<double2 *>(v), 3, c->stream);
     CK(cudaGetLastError());
     return CDNS_OK;
 }
@@ -494,7 +495,7 @@ int cdns_get_velocity(cdns_ctx *c, double *v) {
     int r = cdns_get_velocity_device(c, reinterpret_cast<double *>(c->aux2));
     if (r) return r;
     DeviceGuard guard(c->device);
-    CK(cudaMemcpyAsync(v, c->aux2, sizeof(double2) * 3 * c->d.Ns, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(v, c->aux2, sizeof(double2) * 3 * c->d.Nl, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     return CDNS_OK;
 }
@@ -502,7 +503,9 @@ int cdns_get_velocity(cdns_ctx *c, double *v) {
 int cdns_get_pressure(cdns_ctx *c, double *p) {
     if (!c || !p) return fail(CDNS_ERR_ARG, "null argument");
     DeviceGuard guard(c->device);
-    CK(cudaMemcpyAsync(p, c->p, sizeof(double2) * c->d.Ns, cudaMemcpyDeviceToHost, c->stream));
+    launch_interleave(c->d, c->p, c->aux2, 1, c->stream);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(p, c->aux2, sizeof(double2) * c->d.Nl, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     return CDNS_OK;
 }
@@ -510,7 +513,9 @@ int cdns_get_pressure(cdns_ctx *c, double *p) {
 int cdns_set_pressure(cdns_ctx *c, const double *p) {
     if (!c || !p) return fail(CDNS_ERR_ARG, "null argument");
     DeviceGuard guard(c->device);
-    CK(cudaMemcpyAsync(c->p, p, sizeof(double2) * c->d.Ns, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->aux, p, sizeof(double2) * c->d.Nl, cudaMemcpyHostToDevice, c->stream));
+    launch_deinterleave(c->d, c->aux, c->p, 1, c->stream);
+    CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->stream));
     return CDNS_OK;
 }
@@ -581,13 +586,13 @@ int cdns_nonlinear(cdns_ctx *c, const double *velocity, double *nl, double *pbc)
     if (int r = require_whole(c)) return r;
     DeviceGuard guard(c->device);
     const Dims &d = c->d;
-    CK(cudaMemcpyAsync(c->aux2, velocity, sizeof(double2) * 3 * d.Ns, cudaMemcpyHostToDevice, c->stream));
-    launch_deinterleave(c->aux2, c->aux, d.Ns, 3, c->stream);
+    CK(cudaMemcpyAsync(c->aux2, velocity, sizeof(double2) * 3 * d.Nl, cudaMemcpyHostToDevice, c->stream));
+    launch_deinterleave(d, c->aux2, c->aux, 3, c->stream);
     enqueue_nonlinear(c, c->aux, c->aux2, false, 0);
     launch_pressure_bc(d, c->aux2, c->bw, c->bc_p, c->stream);
-    launch_interleave(c->aux2, c->aux, d.Ns, 3, c->stream);
+    launch_interleave(d, c->aux2, c->aux, 3, c->stream);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(nl, c->aux, sizeof(double2) * 3 * d.Ns, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(nl, c->aux, sizeof(double2) * 3 * d.Nl, cudaMemcpyDeviceToHost, c->stream));
     std::vector<double2> b(2 * (size_t)d.ncol);
     CK(cudaMemcpyAsync(b.data(), c->bc_p, b.size() * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -605,10 +610,10 @@ int cdns_transform_fine(cdns_ctx *c, int dir, const double *in, double *out) {
     if (!c || !in || !out) return fail(CDNS_ERR_ARG, "null argument");
     if (int r = require_whole(c)) return r;
     DeviceGuard guard(c->device);
-    const Dims &d = c->d;
+    const Dims d = planar_dims(c->d);   // the field stays in the reference's order
     const size_t nphys = (size_t)d.NZ2 * d.ny2 * d.NX2;
     if (dir == 'B') {
-        CK(cudaMemcpyAsync(c->aux, in, sizeof(double2) * d.Ns, cudaMemcpyHostToDevice, c->stream));
+        CK(cudaMemcpyAsync(c->aux, in, sizeof(double2) * d.Nl, cudaMemcpyHostToDevice, c->stream));
         launch_ysynth(d, c->t, c->aux, nullptr, 1, 1, c->F, c->stream);
         launch_z_backward(d, c->pz, c->t.root_z, c->F, c->G, 1, c->stream);
         launch_x_c2r(d, c->px, c->t.root_x, c->G, c->phys, c->stream);
@@ -620,7 +625,7 @@ int cdns_transform_fine(cdns_ctx *c, int dir, const double *in, double *out) {
         launch_z_forward(d, c->pz, c->t.root_z, c->H, c->F, 1, c->stream);
         launch_yanalysis(d, c->t, c->F, c->aux, 1, c->stream);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(out, c->aux, sizeof(double2) * d.Ns, cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaMemcpyAsync(out, c->aux, sizeof(double2) * d.Nl, cudaMemcpyDeviceToHost, c->stream));
     } else {
         return fail(CDNS_ERR_ARG, "direction must be 'B' or 'F'");
     }
@@ -651,8 +656,8 @@ int cdns_solve(cdns_ctx *c, double g, const double *rhs, const double *pbc, cons
     double2 *dbv = c->G, *dbp = c->G + 6 * nc;
     CK(cudaMemcpyAsync(dbv, bv.data(), bv.size() * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(dbp, bp.data(), bp.size() * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(c->aux2, rhs, sizeof(double2) * 3 * d.Ns, cudaMemcpyHostToDevice, c->stream));
-    launch_deinterleave(c->aux2, c->aux, d.Ns, 3, c->stream);
+    CK(cudaMemcpyAsync(c->aux2, rhs, sizeof(double2) * 3 * d.Nl, cudaMemcpyHostToDevice, c->stream));
+    launch_deinterleave(d, c->aux2, c->aux, 3, c->stream);
     const double2 *zero = c->zero3;  // zeros for the unused history terms
     StepArgs a{};
     a.u = c->aux;
@@ -671,10 +676,11 @@ int cdns_solve(cdns_ctx *c, double g, const double *rhs, const double *pbc, cons
     a.a0 = 1.0;
     a.solve_only = 1;
     launch_step_solve(d, c->t, c->pp, g, c->st, a, c->stream);
-    launch_interleave(c->aux2, c->aux, d.Ns, 3, c->stream);
+    launch_interleave(d, c->aux2, c->aux, 3, c->stream);
+    launch_interleave(d, c->F, c->H, 1, c->stream);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(velocity, c->aux, sizeof(double2) * 3 * d.Ns, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(pressure, c->F, sizeof(double2) * d.Ns, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(velocity, c->aux, sizeof(double2) * 3 * d.Nl, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(pressure, c->H, sizeof(double2) * d.Nl, cudaMemcpyDeviceToHost, c->stream));
     if (units) CK(cudaMemcpyAsync(units, c->st.unit, sizeof(double) * 2 * d.ncy, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     return CDNS_OK;
@@ -751,16 +757,23 @@ int cdns_debug_copy(cdns_ctx *c, int which, double *out, size_t count) {
     case 6:
     case 7: {
         // stored by their nonzero parts: returned as complex values
-        n = (which == 6 ? 6 : 2) * (size_t)d.Ns;
+        const int nf = which == 6 ? 6 : 2;
+        n = nf * (size_t)d.Nl;
         if (count < 2 * n) return fail(CDNS_ERR_ARG, "debug buffer too small");
-        std::vector<double> h(n);
-        CK(cudaMemcpyAsync(h.data(), which == 6 ? c->st.v_inf : c->st.p_inf, n * sizeof(double),
+        std::vector<double> h(nf * (size_t)d.Ns);
+        CK(cudaMemcpyAsync(h.data(), which == 6 ? c->st.v_inf : c->st.p_inf, h.size() * sizeof(double),
                            cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
-        for (size_t i = 0; i < n; ++i) {
-            const int comp = which == 6 ? (int)((i / (size_t)d.Ns) % 3) : 1;
-            out[2 * i] = inf_imag(comp) ? 0.0 : h[i];
-            out[2 * i + 1] = inf_imag(comp) ? h[i] : 0.0;
+        size_t i = 0;
+        for (int f = 0; f < nf; ++f) {
+            const bool imag = which == 6 && inf_imag(f % 3);
+            for (int kz = 0; kz < d.nkz; ++kz)
+                for (int y = 0; y < d.ncy; ++y)
+                    for (int kx = 0; kx < d.nkx; ++kx, ++i) {
+                        const double v = h[f * (size_t)d.Ns + spectral_base(d, kz, kx) + (size_t)y * d.sy];
+                        out[2 * i] = imag ? 0.0 : v;
+                        out[2 * i + 1] = imag ? v : 0.0;
+                    }
         }
         return CDNS_OK;
     }

@@ -81,9 +81,9 @@ template <typename Fill> int atomic_write(const char *path, Fill fill) {
 
 // The velocity in the reference layout, on the host.
 int velocity_host(cdns_ctx *c, std::vector<double> &v) {
-    const size_t n = 3 * (size_t)c->d.Ns;
+    const size_t n = 3 * (size_t)c->d.Nl;
     v.resize(2 * n);
-    launch_interleave(c->U[c->cur], c->aux, c->d.Ns, 3, c->stream);
+    launch_interleave(c->d, c->U[c->cur], c->aux, 3, c->stream);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(v.data(), c->aux, n * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -172,7 +172,7 @@ int cdns_read_restart(cdns_ctx *c, const char *path, long long *step, double *ti
     std::string t((std::istreambuf_iterator<char>(in)), std::istreambuf_iterator<char>());
     const Dims &d = c->d;
     const cdns_mesh_desc &m = c->mesh;
-    const size_t nvals = 2 * 3 * (size_t)d.Ns;
+    const size_t nvals = 2 * 3 * (size_t)d.Nl;
     std::vector<double> v(nvals);
     long long s = 0;
     double tm = 0.0;

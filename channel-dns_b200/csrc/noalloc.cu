@@ -122,7 +122,7 @@ extern "C" int cdns_transform_fine_backward_noalloc(const cdns_mesh_desc *m, con
     d.fcol = d.ncol;
     d.zc = d.NZS * d.nkx;
     d.nyh = m->NY2 / 2 + 1;
-    d.Ns = (long long)d.nkz * d.ncy * d.nkx;
+    d = planar_dims(d);   // the caller's array is in the reference's order
     FftPlan px{}, pz{};
     if (!factor(d.NX2, px) || !factor(d.NZ2, pz))
         return record_error(CDNS_ERR_ARG, "NX2/NZ2 must factor into primes <= 13");

@@ -83,7 +83,7 @@ k_divergence(Dims d, Tables t, const double2 *__restrict__ u, const double2 *__r
         const int c2 = col0 + l;
         if (c2 >= ncol) continue;
         const int kzi = c2 / nkx, kx = c2 - (c2 / nkx) * nkx;
-        const long long off = ((long long)kzi * ncy + y) * nkx + kx;
+        const long long off = spectral_base(d, kzi, kx) + (long long)y * d.sy;
         tile[tile_slot<E>(y, l)] = u[d.Ns + off];
     }
     __syncthreads();
@@ -108,7 +108,7 @@ k_divergence(Dims d, Tables t, const double2 *__restrict__ u, const double2 *__r
         const int c2 = col0 + l;
         if (c2 >= ncol) continue;
         const int kzi = c2 / nkx, kx = c2 - (c2 / nkx) * nkx;
-        const long long off = ((long long)kzi * ncy + y) * nkx + kx;
+        const long long off = spectral_base(d, kzi, kx) + (long long)y * d.sy;
         const double2 a = u[off], b = u[d.Ns + off], c = u[2 * d.Ns + off], q = p[off];
         ok = ok && isfinite(a.x) && isfinite(a.y) && isfinite(b.x) && isfinite(b.y) && isfinite(c.x) &&
              isfinite(c.y) && isfinite(q.x) && isfinite(q.y);
@@ -456,11 +456,11 @@ int cdns_transform_coarse(cdns_ctx *c, int dir, const double *in, double *out) {
     int r = ensure_output(c, true);
     if (r) return r;
     OutputWork *w = c->outw;
-    const Dims &d = c->d, &dc = w->dc;
+    const Dims dc = planar_dims(w->dc);   // the field stays in the reference's order
     cudaStream_t s = c->stream;
     const size_t nphys = (size_t)dc.NZ2 * dc.ny2 * dc.NX2;
     if (dir == 'B') {
-        CK(cudaMemcpyAsync(w->pd, in, sizeof(double2) * d.Ns, cudaMemcpyHostToDevice, s));
+        CK(cudaMemcpyAsync(w->pd, in, sizeof(double2) * dc.Nl, cudaMemcpyHostToDevice, s));
         launch_ysynth(dc, w->tc, w->pd, nullptr, 1, 1, w->F, s);
         launch_z_backward(dc, w->pz, w->tc.root_z, w->F, w->G, 1, s, true);
         launch_x_c2r(dc, w->px, w->tc.root_x, w->G, w->phys, s, true);
@@ -472,7 +472,7 @@ int cdns_transform_coarse(cdns_ctx *c, int dir, const double *in, double *out) {
         launch_z_forward(dc, w->pz, w->tc.root_z, w->G, w->F, 1, s, true);
         launch_yanalysis(dc, w->tc, w->F, w->pd, 1, s);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(out, w->pd, sizeof(double2) * d.Ns, cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(out, w->pd, sizeof(double2) * dc.Nl, cudaMemcpyDeviceToHost, s));
     } else {
         return fail(CDNS_ERR_ARG, "direction must be 'B' or 'F'");
     }

@@ -134,7 +134,7 @@ Dims slab_dims(const cdns_ctx *c) {
     ds.ncol = ds.nkx * ds.nkz;
     ds.fcol = ds.ncol;
     ds.ny2 = w.nj[w.rank];
-    ds.Ns = (long long)ds.nkz * ds.ncy * ds.nkx;
+    set_tiled(ds);
     return ds;
 }
 

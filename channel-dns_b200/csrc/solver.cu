@@ -14,7 +14,7 @@
 // downward sweep and the wall sums inside the upward one.
 //
 // The influence-matrix and sigma corrections then run over the block as one
-// coalesced elementwise pass over the planar influence and B-problem fields
+// coalesced elementwise pass over the influence and B-problem fields
 // (solver_setup.cu).  Three symmetries cut what that pass reads from twelve
 // real fields to six over the kz <= 0 half:
 //   - the second influence response is the mirror image of the first under
@@ -48,8 +48,8 @@ __device__ __forceinline__ double ld256(const double *p) {
 }
 struct SolveArgs {
     double p_a, p_b;           // pressure wall condition a P + b dP/dn
-    double2 *p_out;            // [Ns] planar
-    double2 *v_out;            // [3][Ns] planar
+    double2 *p_out;            // [Ns]
+    double2 *v_out;            // [3][Ns]
     StepArgs step;
 };
 
@@ -298,7 +298,7 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
     {
         constexpr int kBatch = 2;
         double2 sy = mk(0.0, 0.0);   // N_y over this thread's rows (all of parity g & 1)
-        const long long base = (long long)kzi * ncy * nkx + kx;
+        const long long base = spectral_base(d, kzi, kx);
         for (int y0 = g; ok && y0 < ncy; y0 += kBatch * kRowGroups) {
             double2 u[kBatch][3], up[kBatch][3], nv[kBatch][3], np[kBatch][3];
 #pragma unroll
@@ -306,7 +306,7 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
                 const int y = min(y0 + b * kRowGroups, ny);
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
-                    const long long o = c * d.Ns + base + (long long)y * nkx;
+                    const long long o = c * d.Ns + base + (long long)y * d.sy;
                     u[b][c] = ld256(s.u + o);
                     up[b][c] = ld256(s.u_prev + o);
                     nv[b][c] = ld256(s.N + o);
@@ -373,14 +373,14 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
         }
         tail = T[(2 * S) + (ny - p) * (2 * TC) + own];   // R_1 at ny, ny - 1
         {
-            const long long o_n = ((long long)(coln / nkx) * ncy + ny) * nkx + coln % nkx;
+            const long long o_n = spectral_base(d, coln / nkx, coln % nkx) + (long long)ny * d.sy;
             i00 = st.inf_div[coln].x;
             i01 = st.inf_div[ncol + coln].x;
             i10 = st.inf_div[2 * ncol + coln].x;
             i11 = st.inf_div[3 * ncol + coln].x;
             sg = st.sigma0[p * ncol + coln].x;
             pn = st.p_inf[o_n];
-            vn = st.v_inf[d.Ns + o_n - p * nkx];
+            vn = st.v_inf[d.Ns + o_n - p * d.sy];
         }
         __syncwarp();   // the sums were read by every lane before P's sweep overwrites them
         DivergenceRhs rhs{T + oth, T + 2 * S + own, T + 4 * S + oth, sx, sz, ny};
@@ -480,13 +480,13 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
         const double fu = axl != 0.0 ? 1.0 : 0.0;
         const double fw = same_uw && axl != 0.0 ? azl / axl : sgn;
         const long long comp = axl != 0.0 ? 0 : 2 * d.Ns;
-        const long long in0 = (long long)kzn * ncy * nkx + kx, out0 = (long long)kzi * ncy * nkx + kx;
+        const long long in0 = spectral_base(d, kzn, kx), out0 = spectral_base(d, kzi, kx);
         constexpr int kBatch = 4;
         for (int y0 = g; y0 < ncy; y0 += kBatch * kRowGroups) {
             double pi[kBatch], qi[kBatch], vi[kBatch], wi[kBatch], pb[kBatch], qb[kBatch], vb[kBatch], wb[kBatch];
 #pragma unroll
             for (int k = 0; k < kBatch; ++k) {
-                const long long o = in0 + (long long)min(y0 + k * kRowGroups, ny) * nkx;
+                const long long o = in0 + (long long)min(y0 + k * kRowGroups, ny) * d.sy;
                 pi[k] = ld256(st.p_inf + o);
                 vi[k] = ld256(st.v_inf + d.Ns + o);
                 pb[k] = ld256(st.p_b + o);
@@ -518,7 +518,7 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
                 }
                 bad |= !(isfinite(pr.x) && isfinite(pr.y) && isfinite(v[0].x) && isfinite(v[0].y) &&
                          isfinite(v[1].x) && isfinite(v[1].y) && isfinite(v[2].x) && isfinite(v[2].y));
-                const long long o = out0 + (long long)y * nkx;
+                const long long o = out0 + (long long)y * d.sy;
                 A.p_out[o] = pr;
 #pragma unroll
                 for (int c = 0; c < 3; ++c) A.v_out[c * d.Ns + o] = v[c];
@@ -569,7 +569,7 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
                 u2.x += dpdz * uu[ncy + y];
                 bad |= !(isfinite(pz.x) && isfinite(pz.y) && isfinite(u0.x) && isfinite(u0.y) && isfinite(u1.x) &&
                          isfinite(u1.y) && isfinite(u2.x) && isfinite(u2.y));
-                const long long off = ((long long)d.NZS * ncy + y) * nkx + (zc - d.NZS * nkx);
+                const long long off = spectral_base(d, d.NZS, zc - d.NZS * nkx) + (long long)y * d.sy;
                 A.p_out[off] = pz;
                 A.v_out[off] = u0;
                 A.v_out[d.Ns + off] = u1;
@@ -627,11 +627,11 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
     __syncthreads();
     if (ok) {
         const double axl = t.wavx[kx], azl = t.wavz[kzi];
-        const long long out0 = (long long)kzi * ncy * nkx + kx;
+        const long long out0 = spectral_base(d, kzi, kx);
 #pragma unroll 4
         for (int y = g; y < ncy; y += kRowGroups) {
             const int sl = y * TC + l;
-            const long long o = out0 + (long long)y * nkx;
+            const long long o = out0 + (long long)y * d.sy;
             const double2 v = tile[S + sl];
             const double2 du = y < ny ? tile[sl + TC] : mk(0.0, 0.0), dw = y < ny ? tile[2 * S + sl + TC] : mk(0.0, 0.0);
             s.om[o] = csub(dw, fderiv(azl, v));
@@ -666,10 +666,10 @@ __global__ void k_pressure_bc(Dims d, const double2 *N, const double2 *bw, doubl
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= d.ncol) return;
     const int kzi = col / d.nkx, kx = col - (col / d.nkx) * d.nkx;
-    const double2 *Ny = N + d.Ns + (long long)kzi * d.ncy * d.nkx + kx;
+    const double2 *Ny = N + d.Ns + spectral_base(d, kzi, kx);
     double2 st_ = mk(0, 0), sb_ = mk(0, 0);
     for (int y = 0; y <= d.NYS; ++y) {
-        const double2 n1 = Ny[(long long)y * d.nkx];
+        const double2 n1 = Ny[(long long)y * d.sy];
         st_ = cadd(st_, n1);
         sb_ = (y & 1) ? cadd(sb_, n1) : csub(sb_, n1);
     }

@@ -10,8 +10,8 @@
 // computed in the same order.  Setup runs at steps 1 and 2 only.
 //
 // Outputs: the pivots ad_p, ad_v are stored column-major ([col][y]), read by
-// the step solve's column warps; the influence / B-problem fields are planar
-// ([kz][y][kx]), read by its coalesced correction pass.
+// the step solve's chains; the influence / B-problem fields are in the tiled
+// layout, read by its coalesced correction pass.
 #include "cdns_kernels.cuh"
 
 namespace cdns {
@@ -24,8 +24,8 @@ enum SetupMode { MODE_BASE = 1, MODE_COUPLED = 2 };
 
 struct SetupArgs {
     double2 bcp_top, bcp_bot;  // constant pressure wall data
-    double *p_out;             // [Ns] planar, real
-    double *v_out;             // [3][Ns] planar, parts as inf_imag(c)
+    double *p_out;             // [Ns], real
+    double *v_out;             // [3][Ns], parts as inf_imag(c)
     double2 *divb_out;         // [2][ncol] raw wall divergence (MODE_BASE)
 };
 
@@ -227,7 +227,7 @@ k_setup_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, Setup
         const int col = col0 + l;
         if (col >= nhalf) continue;
         const int kzi = col / nkx, kx = col - (col / nkx) * nkx;
-        const long long cm = ((long long)kzi * ncy + y) * nkx + kx;   // planar
+        const long long cm = spectral_base(d, kzi, kx) + (long long)y * d.sy;
         double2 p = pc[i];
         double2 v[3] = {rv[i], rv[S + i], rv[2 * S + i]};
         if (MODE == MODE_COUPLED) {
@@ -243,7 +243,7 @@ k_setup_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, Setup
         for (int c = 0; c < 3; ++c) A.v_out[c * d.Ns + cm] = vv[c];
         const int kzm = 2 * d.NZS - kzi;
         if (kzm != kzi) {
-            const long long mm = ((long long)kzm * ncy + y) * nkx + kx;
+            const long long mm = spectral_base(d, kzm, kx) + (long long)y * d.sy;
             A.p_out[mm] = pv;
             A.v_out[mm] = vv[0];
             A.v_out[d.Ns + mm] = vv[1];
@@ -313,10 +313,10 @@ __global__ void k_sigma0(Dims d, double re, const double *wn_v, const double *p_
     if (col >= d.ncol) return;
     const int kzi = col / d.nkx, kx = col - (col / d.nkx) * d.nkx;
     const int n = d.NYS;
-    const long long on = ((long long)kzi * d.ncy + n) * d.nkx + kx;   // planar (kz, n, kx)
+    const long long on = spectral_base(d, kzi, kx) + (long long)n * d.sy;
     const double w = wn_v[col];
     const double2 vbn = inf_value(v_b[d.Ns + on], false);
-    const double2 vbn1 = inf_value(v_b[d.Ns + on - d.nkx], false);
+    const double2 vbn1 = inf_value(v_b[d.Ns + on - d.sy], false);
     const double2 pbn = inf_value(p_b[on], false);
     sigma0[col] = mk(re + w * vbn.x, w * vbn.y);
     double2 s1 = csub(mk(re + w * vbn1.x, w * vbn1.y), cscale(re * (2.0 * n), pbn));

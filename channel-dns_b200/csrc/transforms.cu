@@ -268,12 +268,12 @@ k_ydct_r(Dims d, const double2 *__restrict__ roots, const double *__restrict__ c
     double2 xa[NI], xb[NI];
     if (!ANA) {
         const double2 *S = (f < A.nsplit ? A.spec0 + (long long)f * d.Ns : A.spec1 + (long long)(f - A.nsplit) * d.Ns) +
-                           (long long)kzi * ncy * nkx + kx;
+                           spectral_base(d, kzi, kx);
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
             const int n = r + R * i, m = N - n;
-            xa[i] = (n <= N / 2 && n < ncy && lok) ? S[(long long)n * nkx] : mk(0.0, 0.0);
-            xb[i] = (n <= N / 2 && m < ncy && lok) ? S[(long long)m * nkx] : mk(0.0, 0.0);
+            xa[i] = (n <= N / 2 && n < ncy && lok) ? S[(long long)n * d.sy] : mk(0.0, 0.0);
+            xb[i] = (n <= N / 2 && m < ncy && lok) ? S[(long long)m * d.sy] : mk(0.0, 0.0);
         }
     } else {
         const CT *F = A.Fin + (long long)f * d.ny2 * d.fcol + (long long)kzi * nkx + kx;
@@ -335,7 +335,7 @@ k_ydct_r(Dims d, const double2 *__restrict__ roots, const double *__restrict__ c
     CT *Fo = nullptr;
     double2 *So = nullptr;
     if (!ANA) Fo = A.Fout + (long long)f * d.ny2 * d.fcol + (long long)kzi * nkx + kx;
-    else So = A.S + (long long)f * d.Ns + (long long)kzi * ncy * nkx + kx;
+    else So = A.S + (long long)f * d.Ns + spectral_base(d, kzi, kx);
     // mean profile (kz, kx) = (0, 0) of FP32 stages: kept in FP64, out of the
     // FP32 buffer (its imaginary part is round-off of a real profile)
     const bool to_mean = !ANA && A.mean && kzi == d.NZS && kx == 0;
@@ -349,7 +349,7 @@ k_ydct_r(Dims d, const double2 *__restrict__ roots, const double *__restrict__ c
                 Fo[(long long)j * d.fcol] = cto<CT>(cscale(j == 0 || j == N ? A.outE : A.outI, v));
             }
         } else if (j < ncy) {
-            So[(long long)j * nkx] = cscale(j == 0 ? A.s0 : A.sk, v);
+            So[(long long)j * d.sy] = cscale(j == 0 ? A.s0 : A.sk, v);
         }
     };
     // ---- even outputs X_2k = (Z_k + Z_{N-k}) / 2; chunk sums of i (Z_q - Z_{N-q}) / 2

@@ -6,7 +6,7 @@
 // y that couple one parity (Chebyshev derivatives, tau elimination sweeps)
 // become first-order affine recurrences along the 16 lanes of a parity: a
 // sequential pass over a lane's E coefficients, a 4-level shuffle scan, and a
-// carry-in.  Blocks of kColsPerBlock warps stage the planar [kz][y][kx]
+// carry-in.  Blocks of kColsPerBlock warps stage one tile of the
 // spectral layout through swizzled shared-memory tiles so that global
 // accesses are coalesced rows of kColsPerBlock columns.
 #pragma once

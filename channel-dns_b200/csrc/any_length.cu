@@ -151,10 +151,12 @@ k_z_forward_any(Dims d, int N1, int N2, const double2 *__restrict__ roots, const
 // Rows are written where they were read in 2 and 4, so those need no barrier
 // between; SP odd keeps rows and columns free of bank conflicts.
 // ---------------------------------------------------------------------------
-// 16 warps per SM (12 for the 25 instance): at most 128 (168) registers
+// 15 or 16 warps per SM: at most 128 registers.  The 25 instance spills there
+// (484 bytes), but its 10 warps with 168 registers took 1.39 ms for 384 x 289 x
+// 288 points against 1.12.
 __host__ __device__ constexpr int x_threads(int maxr) { return maxr > 20 ? 160 : 128; }
 template <int MAXR>
-__global__ void __launch_bounds__(x_threads(MAXR), MAXR > 20 ? 2 : 4)
+__global__ void __launch_bounds__(x_threads(MAXR), MAXR > 20 ? 3 : 4)
 k_x_cross_any(Dims d, int N1, int N2, int NP, const double2 *__restrict__ roots, const double2 *__restrict__ G,
               double2 *__restrict__ H) {
     extern __shared__ double2 sm_d[];

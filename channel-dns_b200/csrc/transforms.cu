@@ -231,9 +231,9 @@ k_z_forward_peers(Dims d, const double2 *__restrict__ roots, const double2 *__re
 //   the carry of the earlier chunks (a fixed-order sum of their totals) and
 //   the odd outputs, stored from registers.  Stores run along kx (11-16 lines of
 //   one row per thread group), as the loads do.
-// Bound by latency and the shared-memory pipe: at N = 192 the one array leaves 5
-// blocks of 176 threads per SM (41 KB each) where a separate x and Z took 3 of
-// 74 KB, and pairing drops one of seven shared passes.
+// Bound by latency and the shared-memory pipe: at N = 192 the one array leaves
+// room for 5 blocks of 176 threads per SM (41 KB each; the registers, 4) where a
+// separate x and Z took 3 of 74 KB, and pairing drops one of seven shared passes.
 // Shared memory: twiddles [N], the array, partials [16][TL] (Y_1's, then the
 // chunk totals), Y_1 [TL].
 // ---------------------------------------------------------------------------
@@ -242,8 +242,12 @@ __host__ __device__ constexpr size_t ydct_slots(int n1, int n2, int tl) {
     return (size_t)n1 * n2 + (size_t)n1 * fft2_kstride(n2, tl) + (size_t)kYdctRows * tl + tl;
 }
 
+// Blocks per SM that the registers are held to: 24 warps of at most 80 registers
+// (21 at TL = 13, whose blocks take 7 warps).  Left free, TL = 11 took 86 and 3
+// blocks: the synthesis ran in 97 instead of 87 us at Re_tau180.
+__host__ __device__ constexpr int ydct_blocks(int tl) { return tl == 8 ? 6 : tl == 11 ? 4 : 3; }
 template <int N1, int N2, bool ANA, int TL, class CT>
-__global__ void __launch_bounds__(16 * TL)
+__global__ void __launch_bounds__(16 * TL, ydct_blocks(TL))
 k_ydct_r(Dims d, const double2 *__restrict__ roots, const double *__restrict__ cosy, YdctArgs<CT> A) {
     constexpr int N = N1 * N2;
     constexpr int R = kYdctRows;
@@ -1529,8 +1533,8 @@ int z_lines(const Dims &d) {
 template <typename Fn> bool with_xsplit(int nx2, Fn &&fn);
 // kx lines per block of the DCT kernels: of {8, 11, 13, 16}, the width that
 // keeps the most threads per SM on real lines -- blocks per SM by shared
-// memory (228 KB, 1 KB reserved per block) x 16 TL threads x nkx / (nkx
-// padded to TL) -- the wider one on a tie; CDNS_YDCT_LINES fixes it.
+// memory (228 KB, 1 KB reserved per block) and registers (ydct_blocks) x 16 TL
+// threads x nkx / (nkx padded to TL) -- the wider one on a tie; CDNS_YDCT_LINES fixes it.
 int ydct_lines(const Dims &d) {
     const char *e = std::getenv("CDNS_YDCT_LINES");
     const int forced = e ? std::atoi(e) : 0;
@@ -1544,7 +1548,7 @@ int ydct_lines(const Dims &d) {
     double best_useful = -1.0;
     for (int tl : {16, 13, 11, 8}) {
         const size_t bytes = sizeof(double2) * ydct_slots(n1, n2, tl) + 1024;
-        const int blocks = (int)std::min<size_t>((228u * 1024u) / bytes, 2048 / (16 * tl));
+        const int blocks = (int)std::min<size_t>((228u * 1024u) / bytes, ydct_blocks(tl));
         const int padded = ((d.nkx + tl - 1) / tl) * tl;
         const double useful = (double)blocks * 16 * tl * d.nkx / padded;
         if (useful > best_useful) {

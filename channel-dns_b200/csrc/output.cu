@@ -118,48 +118,40 @@ k_divergence(Dims d, Tables t, const double2 *__restrict__ u, const double2 *__r
     if (__any_sync(kFull, !ok) && (tid & 31) == 0) atomicOr(flag, 1u);
 }
 
-// Plane sums of the x-stage partials in a fixed order (one block per plane).
-__global__ void k_plane_finalize(int nblocks, const double *__restrict__ partial, double *__restrict__ planes) {
-    constexpr int K = 22;
-    const int j = blockIdx.x, k = threadIdx.x;
-    if (k >= K) return;
-    const double *p = partial + (long long)j * nblocks * K;
-    double t = p[k];
-    for (int b = 1; b < nblocks; ++b) t = (k == 21) ? fmin(t, p[b * K + k]) : t + p[b * K + k];
-    planes[j * K + k] = t;
-}
-
-// Statistics::accumulate (src/sim/statistics.cpp:117-139) on the device:
-// running means (old * count + sample) / (count + 1) of the plane moments
-// scaled by 1/(NX NZ), in the layout [20][NY+1]:
+// Plane sums of the x-stage partials in a fixed order, one block per plane: 8
+// lanes a slot, combined by shuffles.  With stats (a statistics sample) the block
+// also takes its plane into the running means, Statistics::accumulate
+// (src/sim/statistics.cpp:117-139): (old * count + sample) / (count + 1) of the
+// moments scaled by 1/(NX NZ), in the layout [20][NY+1]:
 //   0-2 velocity mean, 3 pressure mean, 4-9 velocity second moments (uu vv
 //   ww uv vw wu), 10 pressure second, 11-13 pressure-velocity, 14-16
 //   velocity third, 17-19 velocity fourth; then the dpdx and dpdz means.
-__global__ void k_stats_accumulate(int ny1, double scale, long long count, const double *__restrict__ planes,
-                                   const double *__restrict__ dpdx, double *__restrict__ stats) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const double cn = (double)count, cn1 = (double)(count + 1);
-    auto upd = [&](int slot, double sample) {
-        double &o = stats[(long long)slot * ny1 + j];
-        o = (o * cn + sample) / cn1;
-    };
-    if (j < ny1) {
-        const double *sm = planes + (long long)j * 22;
-        upd(3, sm[3] * scale);
-        upd(10, sm[13] * scale);
-        for (int c = 0; c < 3; ++c) {
-            upd(c, sm[c] * scale);
-            upd(4 + c, sm[4 + c] * scale);
-            upd(7 + c, sm[7 + c] * scale);
-            upd(11 + c, sm[10 + c] * scale);
-            upd(14 + c, sm[14 + c] * scale);
-            upd(17 + c, sm[17 + c] * scale);
-        }
+__global__ void __launch_bounds__(192)
+k_plane_finalize(int nblocks, const double *__restrict__ partial, double *__restrict__ planes, int ny1, double scale,
+                 long long count, const double *__restrict__ dpdx, double *__restrict__ stats) {
+    constexpr int K = 22, LANES = 8;
+    const int j = blockIdx.x, k = threadIdx.x / LANES, i = threadIdx.x % LANES;
+    const double *p = partial + (long long)j * nblocks * K + k;
+    double t = k == 21 ? 1.0 : 0.0;
+    if (k < K)
+        for (int b = i; b < nblocks; b += LANES) t = (k == 21) ? fmin(t, p[b * K]) : t + p[b * K];
+#pragma unroll
+    for (int m = LANES / 2; m > 0; m >>= 1) {
+        const double o = __shfl_xor_sync(0xffffffffu, t, m);
+        t = (k == 21) ? fmin(t, o) : t + o;
     }
-    if (j == 0) {
-        double *dm = stats + 20LL * ny1;
-        dm[0] = (dm[0] * cn + dpdx[0]) / cn1;
-        dm[1] = (dm[1] * cn + dpdx[1]) / cn1;
+    if (i != 0 || k >= K) return;
+    planes[j * K + k] = t;
+    if (!stats) return;
+    const double cn = (double)count, cn1 = (double)(count + 1);
+    if (k < 20) {
+        // plane sums: u v w p, uu vv ww, uv vw wu, pu pv pw, pp, u^3.., u^4..
+        const int slot = k == 13 ? 10 : k >= 10 && k < 13 ? k + 1 : k;
+        double &o = stats[(long long)slot * ny1 + j];
+        o = (o * cn + t * scale) / cn1;
+    } else if (j == 0) {   // slots 20 and 21 hold no moment: their threads take dp/dx and dp/dz
+        double *dm = stats + 20LL * ny1 + (k - 20);
+        *dm = (*dm * cn + dpdx[k - 20]) / cn1;
     }
 }
 
@@ -321,7 +313,7 @@ int ensure_output(cdns_ctx *c, bool snapshot) {
 // check = true adds the divergence (sum 20) and the spectral finite check of
 // a check step; a statistics sample needs neither and synthesises u, v, w, p
 // straight from the state.
-int enqueue_reduction(cdns_ctx *c, bool snapshot, bool check) {
+int enqueue_reduction(cdns_ctx *c, bool snapshot, bool check, bool sample = false) {
     OutputWork *w = c->outw;
     const Dims &d = c->d, &dc = w->dc;
     cudaStream_t s = c->stream;
@@ -335,7 +327,9 @@ int enqueue_reduction(cdns_ctx *c, bool snapshot, bool check) {
     const int nf = check ? 5 : 4;
     launch_z_backward(dc, w->pz, w->tc.root_z, w->F, w->G, nf, s, true);
     launch_x_moments(dc, w->px, w->tc.root_x, w->G, w->partial, snapshot ? w->phys : nullptr, nf, s);
-    k_plane_finalize<<<dc.ny2, 32, 0, s>>>(moment_blocks(dc), w->partial, w->planes);
+    k_plane_finalize<<<dc.ny2, 192, 0, s>>>(moment_blocks(dc), w->partial, w->planes, dc.ny2,
+                                            1.0 / ((double)dc.NX2 * (double)dc.NZ2), w->count, c->dpdx,
+                                            sample ? w->stats : nullptr);
     CK(cudaGetLastError());
     return CDNS_OK;
 }
@@ -407,13 +401,8 @@ int cdns_statistics_sample(cdns_ctx *c) {
     if (!c->have_velocity) return fail(CDNS_ERR_STATE, "cdns_statistics_sample before cdns_set_velocity");
     DeviceGuard guard(c->device);
     int r = ensure_output(c, false);
-    if (r || (r = enqueue_reduction(c, false, false))) return r;
+    if (r || (r = enqueue_reduction(c, false, false, true))) return r;
     OutputWork *w = c->outw;
-    const Dims &dc = w->dc;
-    const double scale = 1.0 / ((double)dc.NX2 * (double)dc.NZ2);
-    k_stats_accumulate<<<(dc.ny2 + 127) / 128, 128, 0, c->stream>>>(dc.ny2, scale, w->count, w->planes, c->dpdx,
-                                                                      w->stats);
-    CK(cudaGetLastError());
     ++w->count;
     return CDNS_OK;
 }

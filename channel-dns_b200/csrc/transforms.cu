@@ -1152,6 +1152,7 @@ k_x_adjoint_r(Dims d, const double2 *__restrict__ roots, const double2 *__restri
 // doubled (the coarse c2r convention).
 // ---------------------------------------------------------------------------
 constexpr int kMomentSlots = 22;
+constexpr int kMomentLanes = 8;   // threads that sum one slot (22 x 8 <= the block's threads)
 
 struct MomentAcc {
     double s[21];
@@ -1173,26 +1174,26 @@ struct MomentAcc {
         s[17] += uu * uu; s[18] += vv * vv; s[19] += ww * ww;
         s[20] += dv * dv;
     }
-    // block sum (fixed order) into out[0..21]; red holds 32 x kMomentSlots doubles
+    // Block sums (fixed order) into out[0..21]; red holds kMomentSlots x blockDim.x
+    // doubles.  Every thread leaves its 22 values there, then kMomentLanes threads
+    // a slot sum them and combine by shuffles: a thread has few points, and 22
+    // shuffle trees over its warp cost more than its points.
     __device__ void store(double *red, double *out) {
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-        double f = ok ? 1.0 : 0.0;
+        const int nt = blockDim.x, t = threadIdx.x;
 #pragma unroll
-        for (int k = 0; k < 21; ++k)
-            for (int m = 16; m > 0; m >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], m);
-        for (int m = 16; m > 0; m >>= 1) f = fmin(f, __shfl_xor_sync(0xffffffffu, f, m));
-        if (lane == 0) {
-#pragma unroll
-            for (int k = 0; k < 21; ++k) red[wid * kMomentSlots + k] = s[k];
-            red[wid * kMomentSlots + 21] = f;
-        }
+        for (int k = 0; k < 21; ++k) red[k * nt + t] = s[k];
+        red[21 * nt + t] = ok ? 1.0 : 0.0;
         __syncthreads();
-        if (threadIdx.x < kMomentSlots) {
-            const int k = threadIdx.x;
-            double t = red[k];
-            for (int q = 1; q < nw; ++q) t = (k == 21) ? fmin(t, red[q * kMomentSlots + k]) : t + red[q * kMomentSlots + k];
-            out[k] = t;
+        const int k = t / kMomentLanes, i = t % kMomentLanes;
+        double v = k == 21 ? 1.0 : 0.0;
+        if (k < kMomentSlots)
+            for (int q = i; q < nt; q += kMomentLanes) v = k == 21 ? fmin(v, red[k * nt + q]) : v + red[k * nt + q];
+#pragma unroll
+        for (int m = kMomentLanes / 2; m > 0; m >>= 1) {
+            const double o = __shfl_xor_sync(0xffffffffu, v, m);
+            v = k == 21 ? fmin(v, o) : v + o;
         }
+        if (i == 0 && k < kMomentSlots) out[k] = v;
     }
 };
 
@@ -1205,7 +1206,6 @@ k_x_moments_r(Dims d, const double2 *__restrict__ roots, const double2 *__restri
     constexpr int SP = N2 + 1;
     extern __shared__ double2 sm_d[];
     C *buf = sm_d + n;
-    __shared__ double red[32 * kMomentSlots];
     const int L = 3 * RW;
     const int slot = threadIdx.x >> 4, sub = threadIdx.x & 15;
     const int j = blockIdx.y, z0 = blockIdx.x * RW;
@@ -1282,7 +1282,8 @@ k_x_moments_r(Dims d, const double2 *__restrict__ roots, const double2 *__restri
             phys[3 * fs + o] = b.y;
         }
     }
-    acc.store(red, partial + ((long long)j * gridDim.x + blockIdx.x) * kMomentSlots);
+    __syncthreads();   // the lines were read: their space takes the partial sums
+    acc.store(reinterpret_cast<double *>(buf), partial + ((long long)j * gridDim.x + blockIdx.x) * kMomentSlots);
 }
 
 // Stockham form of k_x_moments_r for any NX.
@@ -1290,7 +1291,6 @@ __global__ void __launch_bounds__(256)
 k_x_moments(Dims d, FftPlan P, const double2 *__restrict__ roots, const double2 *__restrict__ G, int RW,
             double *__restrict__ partial, double *__restrict__ phys, int nf) {
     extern __shared__ double2 sm[];
-    __shared__ double red[32 * kMomentSlots];
     const int n = d.NX2;
     double2 *s_root = sm;
     const int L = 3 * RW;
@@ -1339,7 +1339,8 @@ k_x_moments(Dims d, FftPlan P, const double2 *__restrict__ roots, const double2 
             phys[3 * fs + o] = p1.y;
         }
     }
-    acc.store(red, partial + ((long long)j * gridDim.x + blockIdx.x) * kMomentSlots);
+    __syncthreads();   // the lines were read: their space takes the partial sums
+    acc.store(reinterpret_cast<double *>(a), partial + ((long long)j * gridDim.x + blockIdx.x) * kMomentSlots);
 }
 
 // ---------------------------------------------------------------------------
@@ -1602,9 +1603,11 @@ constexpr int kRWm = 4;    // rows per block of the output-reduction x stage
 size_t smem_xmoments_r(int n1, int n2) {
     const size_t L = 3 * kRWm;
     const size_t s1 = L * n1 * (n2 + 1), s2 = L * n1 * n2;
-    return sizeof(double2) * (n1 * n2 + (s1 > s2 ? s1 : s2));
+    return sizeof(double2) * (n1 * n2 + std::max(std::max(s1, s2), (size_t)kMomentSlots * 16 * 3 * kRWm / 2));
 }
-size_t smem_xmoments(const Dims &d) { return sizeof(double2) * (size_t)d.NX2 * (1 + 2 * 3 * kRWm); }
+size_t smem_xmoments(const Dims &d) {
+    return sizeof(double2) * ((size_t)d.NX2 + std::max((size_t)d.NX2 * 2 * 3 * kRWm, (size_t)kMomentSlots * 256 / 2));
+}
 size_t smem_zfft_r(const Dims &d, int n1, int n2, size_t elem) {
     // twiddles, then the exchange of fft2_lines: n1 rows of the padded k1 stride
     return sizeof(double2) * n1 * n2 + elem * ((size_t)n1 * fft2_kstride(n2, z_lines(d)));

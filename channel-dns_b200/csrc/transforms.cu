@@ -1152,6 +1152,8 @@ k_x_adjoint_r(Dims d, const double2 *__restrict__ roots, const double2 *__restri
 // doubled (the coarse c2r convention).
 // ---------------------------------------------------------------------------
 constexpr int kMomentSlots = 22;
+// rows per block of k_x_moments_r: 12 lines
+__host__ __device__ constexpr int moment_rows(int lpr) { return 12 / lpr; }
 constexpr int kMomentLanes = 8;   // threads that sum one slot (22 x 8 <= the block's threads)
 
 struct MomentAcc {
@@ -1197,16 +1199,18 @@ struct MomentAcc {
     }
 };
 
-template <int N1, int N2>
-__global__ void __launch_bounds__(16 * 3 * 4)
-k_x_moments_r(Dims d, const double2 *__restrict__ roots, const double2 *__restrict__ G, int RW,
-              double *__restrict__ partial, double *__restrict__ phys, int nf) {
+// LPR lines per row: 3 with the divergence (nf = 5), 2 without; 12 / LPR rows per block.
+template <int N1, int N2, int LPR>
+__global__ void __launch_bounds__(16 * 12)
+k_x_moments_r(Dims d, const double2 *__restrict__ roots, const double2 *__restrict__ G,
+              double *__restrict__ partial, double *__restrict__ phys) {
+    constexpr int RW = moment_rows(LPR), nf = LPR == 3 ? 5 : 4;
     using C = double2;
     constexpr int n = N1 * N2;
     constexpr int SP = N2 + 1;
     extern __shared__ double2 sm_d[];
     C *buf = sm_d + n;
-    const int L = 3 * RW;
+    constexpr int L = LPR * RW;
     const int slot = threadIdx.x >> 4, sub = threadIdx.x & 15;
     const int j = blockIdx.y, z0 = blockIdx.x * RW;
     const int nkx = d.nkx, nxs = d.NXS;
@@ -1217,7 +1221,7 @@ k_x_moments_r(Dims d, const double2 *__restrict__ roots, const double2 *__restri
     C v[N1 > N2 ? N1 : N2];
     const bool act1 = slot < L && sub < N2;
     if (act1) {
-        const int r = slot / 3, q = slot - (slot / 3) * 3;
+        const int r = slot / LPR, q = slot - (slot / LPR) * LPR;
         const int z = z0 + r;
         const C *rowA = Gj + (long long)z * nkx + (2 * q) * fstride;
         const C *rowB = rowA + fstride;
@@ -1272,8 +1276,8 @@ k_x_moments_r(Dims d, const double2 *__restrict__ roots, const double2 *__restri
         const int r = i / n, x = i - (i / n) * n;
         const int z = z0 + r;
         if (z >= d.NZ2) continue;
-        const C a = buf[(3 * r) * n + x], b = buf[(3 * r + 1) * n + x], c = buf[(3 * r + 2) * n + x];
-        acc.add(a.x, a.y, b.x, b.y, c.x);
+        const C a = buf[(LPR * r) * n + x], b = buf[(LPR * r + 1) * n + x];
+        acc.add(a.x, a.y, b.x, b.y, LPR == 3 ? buf[(LPR * r + LPR - 1) * n + x].x : 0.0);
         if (phys) {
             const long long o = ((long long)z * ny1 + j) * n + x, fs = (long long)d.NZ2 * ny1 * n;
             phys[o] = a.x;
@@ -1636,7 +1640,8 @@ template <class C> cudaError_t configure_register_forms(const Dims &d) {
         if (e == cudaSuccess)
             e = raise_smem(k_x_cross_h<N1, N2, C, sizeof(C) == 8>, smem_xcross_h(N1, N2, sizeof(C)));
         if (e == cudaSuccess && sizeof(C) == 16) e = raise_smem(k_x_adjoint_r<N1, N2>, smem_xadjoint_r(N1, N2));
-        if (e == cudaSuccess && sizeof(C) == 16) e = raise_smem(k_x_moments_r<N1, N2>, smem_xmoments_r(N1, N2));
+        if (e == cudaSuccess && sizeof(C) == 16) e = raise_smem(k_x_moments_r<N1, N2, 3>, smem_xmoments_r(N1, N2));
+        if (e == cudaSuccess && sizeof(C) == 16) e = raise_smem(k_x_moments_r<N1, N2, 2>, smem_xmoments_r(N1, N2));
     });
     if (e != cudaSuccess) return e;
     with_xsplit(d.NZ2, [&](auto a, auto b) {
@@ -1904,15 +1909,21 @@ bool launch_ydct_analysis_fp32(const Dims &d, const Tables &t, const float2 *F, 
     return ydct(d, t, nf, true, A, s);
 }
 
-int moment_blocks(const Dims &d) { return (d.NZ2 + kRWm - 1) / kRWm; }
+// x-stage blocks per plane of the output reduction for nf fields
+int moment_blocks(const Dims &d, int nf) {
+    const bool reg = with_xsplit(d.NX2, [](auto, auto) {});
+    const int rw = reg ? moment_rows(nf == 5 ? 3 : 2) : kRWm;
+    return (d.NZ2 + rw - 1) / rw;
+}
 
 void launch_x_moments(const Dims &d, const FftPlan &P, const double2 *roots, const double2 *G, double *partial,
                       double *phys, int nf, cudaStream_t s) {
-    dim3 grid(moment_blocks(d), d.ny2);
+    dim3 grid(moment_blocks(d, nf), d.ny2);
     const bool reg = with_xsplit(d.NX2, [&](auto a, auto b) {
         constexpr int N1 = decltype(a)::value, N2 = decltype(b)::value;
-        k_x_moments_r<N1, N2><<<grid, 16 * 3 * kRWm, smem_xmoments_r(N1, N2), s>>>(d, roots, G, kRWm, partial, phys,
-                                                                                 nf);
+        const size_t sm = smem_xmoments_r(N1, N2);
+        if (nf == 5) k_x_moments_r<N1, N2, 3><<<grid, 16 * 12, sm, s>>>(d, roots, G, partial, phys);
+        else k_x_moments_r<N1, N2, 2><<<grid, 16 * 12, sm, s>>>(d, roots, G, partial, phys);
     });
     if (reg) return;
     k_x_moments<<<grid, 256, smem_xmoments(d), s>>>(d, P, roots, G, kRWm, partial, phys, nf);

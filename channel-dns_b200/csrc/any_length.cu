@@ -105,11 +105,14 @@ __device__ __forceinline__ void fft2_any(int N1, int N2, int TL, const Twiddles<
     });
 }
 
-// threads per block: with the registers of the instance, 18 or 12 warps per SM in
-// two blocks, so that one block's loads overlap the other's DFTs
+// threads per block; 18 warps per SM of at most 96 registers in every instance (with
+// the 160 that the larger ones take when left free, 12 warps: 162 lines-and-rows 97
+// and 63 us instead of 78 and 52, 288 424 and 222 instead of 338 and 191, although
+// the 25 instance spills a kilobyte)
 __host__ __device__ constexpr int z_threads(int maxr) { return maxr > 16 ? 192 : 272; }
+__host__ __device__ constexpr int z_blocks(int maxr) { return maxr > 16 ? 3 : 2; }
 template <int MAXR>
-__global__ void __launch_bounds__(z_threads(MAXR), 2)
+__global__ void __launch_bounds__(z_threads(MAXR), z_blocks(MAXR))
 k_z_backward_any(Dims d, int N1, int N2, const double2 *__restrict__ roots, const double2 *__restrict__ F,
                  double2 *__restrict__ G, int TL, bool coarse) {
     extern __shared__ double2 sm_d[];
@@ -121,7 +124,7 @@ k_z_backward_any(Dims d, int N1, int N2, const double2 *__restrict__ roots, cons
     fft2_any<MAXR, +1>(N1, N2, TL, tw, sm_d + n, src, dst);
 }
 template <int MAXR>
-__global__ void __launch_bounds__(z_threads(MAXR), 2)
+__global__ void __launch_bounds__(z_threads(MAXR), z_blocks(MAXR))
 k_z_forward_any(Dims d, int N1, int N2, const double2 *__restrict__ roots, const double2 *__restrict__ H,
                 double2 *__restrict__ F, int TL, bool coarse) {
     extern __shared__ double2 sm_d[];
@@ -151,12 +154,13 @@ k_z_forward_any(Dims d, int N1, int N2, const double2 *__restrict__ roots, const
 // Rows are written where they were read in 2 and 4, so those need no barrier
 // between; SP odd keeps rows and columns free of bank conflicts.
 // ---------------------------------------------------------------------------
-// 15 or 16 warps per SM: at most 128 registers.  The 25 instance spills there
-// (484 bytes), but its 10 warps with 168 registers took 1.39 ms for 384 x 289 x
-// 288 points against 1.12.
+// 18 to 20 warps per SM of at most 96 registers (176 and 380 bytes spilled), 15 of
+// 128 in the 25 instance (484): warps count for more than spills here.  With 15 of
+// 128 the smaller instances took 271 instead of 251 us at 240 points and 216 instead
+// of 196 at 200; with 10 of 168 the 25 instance took 1.39 ms at 384 instead of 1.12.
 __host__ __device__ constexpr int x_threads(int maxr) { return maxr > 20 ? 160 : 128; }
 template <int MAXR>
-__global__ void __launch_bounds__(x_threads(MAXR), MAXR > 20 ? 3 : 4)
+__global__ void __launch_bounds__(x_threads(MAXR), MAXR > 20 ? 3 : 5)
 k_x_cross_any(Dims d, int N1, int N2, int NP, const double2 *__restrict__ roots, const double2 *__restrict__ G,
               double2 *__restrict__ H) {
     extern __shared__ double2 sm_d[];
@@ -292,10 +296,13 @@ k_x_cross_any(Dims d, int N1, int N2, int NP, const double2 *__restrict__ roots,
 // N2) row groups of TL lines; thread t owns line t mod TL and row group t / TL.
 // ---------------------------------------------------------------------------
 constexpr int kYThreads = 256;
+// blocks of kYThreads per SM that the registers are held to: 24 warps of 80 with
+// factors up to 16 (181 points: 138 us a synthesis, 148 with 16 warps), else 16 of 128
+__host__ __device__ constexpr int y_blocks(int maxr) { return maxr > 16 ? 2 : 3; }
 constexpr int kYPairs = 4;     // pairs of rows of a thread in flight
 constexpr int kYChunk = 13;    // (N/2 + 1) / R, rounded up, is at most this for N1, N2 <= 25
 template <int MAXR, bool ANA, class CT>
-__global__ void __launch_bounds__(kYThreads, MAXR > 20 ? 1 : 2)
+__global__ void __launch_bounds__(kYThreads, y_blocks(MAXR))
 k_ydct_any(Dims d, int N1, int N2, int TL, int R, const double2 *__restrict__ roots,
            const double *__restrict__ cosy, YdctArgs<CT> A) {
     const int N = N1 * N2;
@@ -488,7 +495,8 @@ int y_lines(const Dims &d, int n1, int n2) {
     double best_useful = -1.0;
     for (int tl : {16, 13, 11, 8}) {
         if (R * tl > kYThreads) continue;
-        const int blocks = (int)std::min<size_t>((228u * 1024u) / (smem_y(n1, n2, tl) + 1024), 2048 / (R * tl));
+        const int blocks = (int)std::min<size_t>((228u * 1024u) / (smem_y(n1, n2, tl) + 1024),
+                                                 y_blocks(instance(n1, n2)) * kYThreads / (R * tl));
         const int padded = ((d.nkx + tl - 1) / tl) * tl;
         const double useful = (double)blocks * R * tl * d.nkx / padded;
         if (useful > best_useful) {

@@ -115,6 +115,7 @@ template <int MAXR>
 __global__ void __launch_bounds__(z_threads(MAXR), z_blocks(MAXR))
 k_z_backward_any(Dims d, int N1, int N2, const double2 *__restrict__ roots, const double2 *__restrict__ F,
                  double2 *__restrict__ G, int TL, bool coarse) {
+    chain_begin();
     extern __shared__ double2 sm_d[];
     const int n = N1 * N2;
     const int f = blockIdx.z, j = blockIdx.y, kx0 = blockIdx.x * TL;
@@ -127,6 +128,7 @@ template <int MAXR>
 __global__ void __launch_bounds__(z_threads(MAXR), z_blocks(MAXR))
 k_z_forward_any(Dims d, int N1, int N2, const double2 *__restrict__ roots, const double2 *__restrict__ H,
                 double2 *__restrict__ F, int TL, bool coarse) {
+    chain_begin();
     extern __shared__ double2 sm_d[];
     const int n = N1 * N2;
     const int f = blockIdx.z, j = blockIdx.y, kx0 = blockIdx.x * TL;
@@ -163,6 +165,7 @@ template <int MAXR>
 __global__ void __launch_bounds__(x_threads(MAXR), MAXR > 20 ? 3 : 5)
 k_x_cross_any(Dims d, int N1, int N2, int NP, const double2 *__restrict__ roots, const double2 *__restrict__ G,
               double2 *__restrict__ H) {
+    chain_begin();
     extern __shared__ double2 sm_d[];
     const int n = N1 * N2, SP = N2 | 1, LS = N1 * SP;
     const int T = N1 > N2 ? N1 : N2;
@@ -305,6 +308,7 @@ template <int MAXR, bool ANA, class CT>
 __global__ void __launch_bounds__(kYThreads, y_blocks(MAXR))
 k_ydct_any(Dims d, int N1, int N2, int TL, int R, const double2 *__restrict__ roots,
            const double *__restrict__ cosy, YdctArgs<CT> A) {
+    chain_begin();
     const int N = N1 * N2;
     const int KS = fft2_kstride(N2, TL);
     const int M = N / 2 - 1;               // odd outputs beyond Y_1: k = 1..M
@@ -551,8 +555,8 @@ bool launch_z_any(const Dims &d, const double2 *roots, const double2 *in, double
     const size_t sm = smem_z(a, b, tl);
     with_instance(a, b, [&](auto r) {
         constexpr int M = decltype(r)::value;
-        if (backward) k_z_backward_any<M><<<grid, t * tl, sm, s>>>(d, a, b, roots, in, out, tl, coarse);
-        else k_z_forward_any<M><<<grid, t * tl, sm, s>>>(d, a, b, roots, in, out, tl, coarse);
+        if (backward) launch_chained(k_z_backward_any<M>, grid, t * tl, sm, s, d, a, b, roots, in, out, tl, coarse);
+        else launch_chained(k_z_forward_any<M>, grid, t * tl, sm, s, d, a, b, roots, in, out, tl, coarse);
     });
     return true;
 }
@@ -563,7 +567,7 @@ bool launch_x_cross_any(const Dims &d, const double2 *roots, const double2 *G, d
     const int t = std::max(a, b), np = x_pairs(a, b);
     dim3 grid((d.NZ2 + 2 * np - 1) / (2 * np), d.ny2);
     with_instance(a, b, [&](auto r) {
-        k_x_cross_any<decltype(r)::value><<<grid, 6 * np * t, smem_x(a, b), s>>>(d, a, b, np, roots, G, H);
+        launch_chained(k_x_cross_any<decltype(r)::value>, grid, 6 * np * t, smem_x(a, b), s, d, a, b, np, roots, G, H);
     });
     return true;
 }
@@ -577,8 +581,8 @@ bool launch_ydct_any(const Dims &d, const Tables &t, int nf, bool ana, const Ydc
     const size_t sm = smem_y(a, b, tl);
     with_instance(a, b, [&](auto r) {
         constexpr int M = decltype(r)::value;
-        if (ana) k_ydct_any<M, true, CT><<<grid, R * tl, sm, s>>>(d, a, b, tl, R, t.root_y, t.cosy, A);
-        else k_ydct_any<M, false, CT><<<grid, R * tl, sm, s>>>(d, a, b, tl, R, t.root_y, t.cosy, A);
+        if (ana) launch_chained(k_ydct_any<M, true, CT>, grid, R * tl, sm, s, d, a, b, tl, R, t.root_y, t.cosy, A);
+        else launch_chained(k_ydct_any<M, false, CT>, grid, R * tl, sm, s, d, a, b, tl, R, t.root_y, t.cosy, A);
     });
     return true;
 }

@@ -137,6 +137,34 @@ template <class K> inline cudaError_t raise_smem(K *kernel, size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// Launches of a step follow each other on one stream, each reading what the one
+// before wrote.  launch_chained marks the kernel as a programmatic dependent: its
+// blocks may be set up while the last blocks of the kernel before still run, and
+// chain_begin (the first statement of every kernel launched so) waits for that
+// kernel's end and its writes.  The kernel before the previous one has ended then,
+// too: the previous one waited for it.  No kernel lets its successor in earlier
+// (griddepcontrol.launch_dependents): waiting blocks then hold shared memory that
+// other streams' kernels could use (three 32^3 channels side by side: 18.2 us a
+// step with it, 17.3 without, 17.8 with plain launches; 64^3: 39 us against 42;
+// the allocation-free transform at 72^3, 19.6 us against 26.6).
+template <class... P, class... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Asynchronous global -> shared copies (cp.async, sm_80 and later): 16 bytes
 // cached in L2 only, or 8 bytes; src_bytes below the size fills the rest
 // with zeros (0: zeros only, the source is not read).

@@ -97,6 +97,7 @@ template <int E>
 __global__ void __launch_bounds__(32 * kColsPerBlock)
 k_curl(Dims d, Tables t, const double2 *__restrict__ u, double2 *__restrict__ om,
        double2 *__restrict__ bw, double re) {
+    chain_begin();
     extern __shared__ double2 tile[];   // [3][ncy][kColsPerBlock]
     const int ncy = d.ncy, ny = d.NYS, nkx = d.nkx, ncol = d.ncol;
     const int S = ncy * kColsPerBlock;
@@ -216,6 +217,7 @@ template <class CO>
 __global__ void __launch_bounds__(32 * 2 * kSynTiles, 2)
 k_ysynth(Dims d, const double *__restrict__ csyn, int jp, const double2 *__restrict__ src0,
          const double2 *__restrict__ src1, int nsplit, CO *__restrict__ F, double *__restrict__ mean) {
+    chain_begin();
     extern __shared__ double2 sm[];
     constexpr int KC = kSynKC, KH = KC / 2;
     constexpr int jw = kSynTiles * 16;   // cosine columns staged per block
@@ -346,6 +348,7 @@ template <class CI>
 __global__ void __launch_bounds__(32 * 2 * kMaxGroups)
 k_yanalysis(Dims d, const double *__restrict__ cana, int kh, const CI *__restrict__ F,
             double2 *__restrict__ S, double s0, double sn) {
+    chain_begin();
     // staged complex row of 32 columns: 34 slots for FP64, 36 for FP32 (16-byte units)
     constexpr bool F32 = sizeof(CI) == 8;
     constexpr int XS = F32 ? 36 : kXS;
@@ -455,6 +458,7 @@ k_yanalysis(Dims d, const double *__restrict__ cana, int kh, const CI *__restric
 // memory; one warp per (component, coefficient) sums them.
 __global__ void k_mean_products(Dims d, const double *__restrict__ cana, int kh, const double *__restrict__ mean,
                                 double2 *__restrict__ S) {
+    chain_begin();
     extern __shared__ double sp[];   // [3][NY2+1]
     const int N = d.NY2, ny2 = d.ny2;
     for (int j = threadIdx.x; j < ny2; j += blockDim.x) {
@@ -552,10 +556,10 @@ void launch_curl(const Dims &d, const Tables &t, const double2 *u, double2 *om, 
     const int blocks = (d.ncol + kColsPerBlock - 1) / kColsPerBlock;
     const size_t sm = curl_smem(d);
     switch (lane_elems(d)) {
-    case 1: k_curl<1><<<blocks, 32 * kColsPerBlock, sm, s>>>(d, t, u, om, bw, re); break;
-    case 2: k_curl<2><<<blocks, 32 * kColsPerBlock, sm, s>>>(d, t, u, om, bw, re); break;
-    case 4: k_curl<4><<<blocks, 32 * kColsPerBlock, sm, s>>>(d, t, u, om, bw, re); break;
-    case 8: k_curl<8><<<blocks, 32 * kColsPerBlock, sm, s>>>(d, t, u, om, bw, re); break;
+    case 1: launch_chained(k_curl<1>, blocks, 32 * kColsPerBlock, sm, s, d, t, u, om, bw, re); break;
+    case 2: launch_chained(k_curl<2>, blocks, 32 * kColsPerBlock, sm, s, d, t, u, om, bw, re); break;
+    case 4: launch_chained(k_curl<4>, blocks, 32 * kColsPerBlock, sm, s, d, t, u, om, bw, re); break;
+    case 8: launch_chained(k_curl<8>, blocks, 32 * kColsPerBlock, sm, s, d, t, u, om, bw, re); break;
     default: break;
     }
 }
@@ -566,7 +570,7 @@ void ysynth(const Dims &d, const Tables &t, const double2 *src0, const double2 *
     const int g = syn_groups(d);
     dim3 block(32, 2 * std::min(g, kSynTiles));
     dim3 grid((d.ncol + 31) / 32, nf, (g + kSynTiles - 1) / kSynTiles);
-    k_ysynth<CO><<<grid, block, syn_smem(d), s>>>(d, t.csyn, g * kSynRows, src0, src1, nsplit, F, mean);
+    launch_chained(k_ysynth<CO>, grid, block, syn_smem(d), s, d, t.csyn, g * kSynRows, src0, src1, nsplit, F, mean);
 }
 void launch_ysynth(const Dims &d, const Tables &t, const double2 *src0, const double2 *src1, int nsplit,
                    int nf, double2 *F, cudaStream_t s) {
@@ -585,7 +589,7 @@ void yanalysis(const Dims &d, const double *cana, const CI *F, double2 *S, int n
     const int g = ana_groups(d);
     dim3 block(32, 2 * std::min(g, kMaxGroups));
     dim3 grid((d.ncol + 31) / 32, nf, (g + kMaxGroups - 1) / kMaxGroups);
-    k_yanalysis<CI><<<grid, block, ana_smem(d, sizeof(CI)), s>>>(d, cana, g * kAnaRows, F, S, s0, sn);
+    launch_chained(k_yanalysis<CI>, grid, block, ana_smem(d, sizeof(CI)), s, d, cana, g * kAnaRows, F, S, s0, sn);
 }
 // Output scales of the analysis: s_0 = 1/(2N), s_k = 1/N; FP32 stage buffers
 // arrive without the 1/(NX2 NZ2) of the x and z analyses.
@@ -610,8 +614,7 @@ void launch_yanalysis_scaled(const Dims &d, const double *cana, const double2 *F
 
 void launch_mean_products(const Dims &d, const Tables &t, const double *mean, double2 *S, cudaStream_t s) {
     const int warps = 3 * d.ncy, per_block = 8;
-    k_mean_products<<<(warps + per_block - 1) / per_block, 32 * per_block, sizeof(double) * 3 * d.ny2, s>>>(
-        d, t.cana, ana_groups(d) * kAnaRows, mean, S);
+    launch_chained(k_mean_products, (warps + per_block - 1) / per_block, 32 * per_block, sizeof(double) * 3 * d.ny2, s, d, t.cana, ana_groups(d) * kAnaRows, mean, S);
 }
 
 }  // namespace cdns

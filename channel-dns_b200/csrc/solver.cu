@@ -256,6 +256,7 @@ template <int C> struct VelocityRhs {
 
 __global__ void __launch_bounds__(kThreads, 3)
 k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A) {
+    chain_begin();
     extern __shared__ double2 tile[];   // [4][ncy][TC]: R_0, R_1, R_2, P; then (WL, WR) and the pivots
     __shared__ double s_wall[3][2][2 * TC];
     __shared__ double2 s_cs[TC], s_cd[TC], s_sg[2][TC];   // c0 + c1, c0 - c1, sigma
@@ -700,7 +701,7 @@ void launch_step_solve(const Dims &d, const Tables &t, const PhysParams &pp, dou
     A.v_out = a.u_out;
     A.step = a;
     const int blocks = (d.ncol + TC - 1) / TC;
-    k_solve<<<blocks, kThreads, solve_smem(d), s>>>(d, t, pp, g_v, st, A);
+    launch_chained(k_solve, blocks, kThreads, solve_smem(d), s, d, t, pp, g_v, st, A);
 }
 
 }  // namespace cdns

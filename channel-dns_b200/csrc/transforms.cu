@@ -30,6 +30,7 @@ namespace cdns {
 __global__ void __launch_bounds__(256, 2)
 k_z_backward(Dims d, FftPlan P, const double2 *__restrict__ roots, const double2 *__restrict__ F,
              double2 *__restrict__ G, int TL, bool coarse) {
+    chain_begin();
     extern __shared__ double2 sm[];
     const int n = d.NZ2;
     double2 *s_root = sm;
@@ -46,6 +47,7 @@ k_z_backward(Dims d, FftPlan P, const double2 *__restrict__ roots, const double2
 __global__ void __launch_bounds__(256, 2)
 k_z_forward(Dims d, FftPlan P, const double2 *__restrict__ roots, const double2 *__restrict__ H,
             double2 *__restrict__ F, int TL, bool coarse) {
+    chain_begin();
     extern __shared__ double2 sm[];
     const int n = d.NZ2;
     double2 *s_root = sm;
@@ -115,6 +117,7 @@ template <int N1, int N2, class C>
 __global__ void __launch_bounds__(16 * 17)
 k_z_backward_r(Dims d, const double2 *__restrict__ roots, const C *__restrict__ F, C *__restrict__ G, int TL,
                bool coarse) {
+    chain_begin();
     extern __shared__ double2 sm_d[];
     constexpr int n = N1 * N2;
     C *S = reinterpret_cast<C *>(sm_d + n);
@@ -129,6 +132,7 @@ template <int N1, int N2, class C>
 __global__ void __launch_bounds__(16 * 17)
 k_z_forward_r(Dims d, const double2 *__restrict__ roots, const C *__restrict__ H, C *__restrict__ F, int TL,
               bool coarse) {
+    chain_begin();
     extern __shared__ double2 sm_d[];
     constexpr int n = N1 * N2;
     C *S = reinterpret_cast<C *>(sm_d + n);
@@ -176,6 +180,7 @@ struct ZTruncPeers {
 template <int N1, int N2>
 __global__ void __launch_bounds__(16 * 17)
 k_z_backward_peers(Dims d, const double2 *__restrict__ roots, PeerCols pc, double2 *__restrict__ G, int TL) {
+    chain_begin();
     extern __shared__ double2 sm_d[];
     constexpr int n = N1 * N2;
     double2 *S = sm_d + n;
@@ -189,6 +194,7 @@ k_z_backward_peers(Dims d, const double2 *__restrict__ roots, PeerCols pc, doubl
 template <int N1, int N2>
 __global__ void __launch_bounds__(16 * 17)
 k_z_forward_peers(Dims d, const double2 *__restrict__ roots, const double2 *__restrict__ H, PeerCols pc, int TL) {
+    chain_begin();
     extern __shared__ double2 sm_d[];
     constexpr int n = N1 * N2;
     double2 *S = sm_d + n;
@@ -249,6 +255,7 @@ __host__ __device__ constexpr int ydct_blocks(int tl) { return tl == 8 ? 6 : tl 
 template <int N1, int N2, bool ANA, int TL, class CT>
 __global__ void __launch_bounds__(16 * TL, ydct_blocks(TL))
 k_ydct_r(Dims d, const double2 *__restrict__ roots, const double *__restrict__ cosy, YdctArgs<CT> A) {
+    chain_begin();
     constexpr int N = N1 * N2;
     constexpr int R = kYdctRows;
     constexpr int KS = fft2_kstride(N2, TL);
@@ -397,6 +404,7 @@ k_ydct_r(Dims d, const double2 *__restrict__ roots, const double *__restrict__ c
 __global__ void __launch_bounds__(256, 2)
 k_x_cross(Dims d, FftPlan P, const double2 *__restrict__ roots, const double2 *__restrict__ G,
           double2 *__restrict__ H, int RW) {
+    chain_begin();
     extern __shared__ double2 sm[];
     const int n = d.NX2;
     double2 *s_root = sm;
@@ -514,6 +522,7 @@ template <int N1, int N2, class C, bool MEAN, bool SPLIT = false>
 __global__ void __launch_bounds__(16 * 3 * 4, sizeof(C) == 16 ? 3 : 0)
 k_x_cross_r(Dims d, const double2 *__restrict__ roots, const C *__restrict__ G, C *__restrict__ H, int RW,
             const double *__restrict__ mean) {
+    chain_begin();
     using T = typename CReal<C>::T;
     constexpr int n = N1 * N2;
     constexpr int SP = N2 + 1;   // padded row of the step-1 output
@@ -842,6 +851,7 @@ template <int N1, int N2, class C, bool MEAN>
 __global__ void __launch_bounds__(32 * kXHWarps)
 k_x_cross_h(Dims d, const double2 *__restrict__ roots, const C *__restrict__ G, C *__restrict__ H,
             const double *__restrict__ mean) {
+    chain_begin();
     using T = typename CReal<C>::T;
     constexpr int n = N1 * N2;
     constexpr int NV = N1 > N2 ? N1 : N2;
@@ -1004,6 +1014,7 @@ template <int N1, int N2>
 __global__ void __launch_bounds__(16 * 5 * 2)
 k_x_adjoint_r(Dims d, const double2 *__restrict__ roots, const double2 *__restrict__ G, double2 *__restrict__ Lb,
               int RW) {
+    chain_begin();
     using C = double2;
     constexpr int n = N1 * N2;
     constexpr int SP = N2 + 1;
@@ -1204,6 +1215,7 @@ template <int N1, int N2, int LPR>
 __global__ void __launch_bounds__(16 * 12)
 k_x_moments_r(Dims d, const double2 *__restrict__ roots, const double2 *__restrict__ G,
               double *__restrict__ partial, double *__restrict__ phys) {
+    chain_begin();
     constexpr int RW = moment_rows(LPR), nf = LPR == 3 ? 5 : 4;
     using C = double2;
     constexpr int n = N1 * N2;
@@ -1294,6 +1306,7 @@ k_x_moments_r(Dims d, const double2 *__restrict__ roots, const double2 *__restri
 __global__ void __launch_bounds__(256)
 k_x_moments(Dims d, FftPlan P, const double2 *__restrict__ roots, const double2 *__restrict__ G, int RW,
             double *__restrict__ partial, double *__restrict__ phys, int nf) {
+    chain_begin();
     extern __shared__ double2 sm[];
     const int n = d.NX2;
     double2 *s_root = sm;
@@ -1354,6 +1367,7 @@ k_x_moments(Dims d, FftPlan P, const double2 *__restrict__ roots, const double2 
 __global__ void __launch_bounds__(128)
 k_x_c2r(Dims d, FftPlan P, const double2 *__restrict__ roots, const double2 *__restrict__ G,
         double *__restrict__ phys, int RW, double nyq_scale) {
+    chain_begin();
     extern __shared__ double2 sm[];
     const int n = d.NX2;
     double2 *s_root = sm;
@@ -1394,6 +1408,7 @@ k_x_c2r(Dims d, FftPlan P, const double2 *__restrict__ roots, const double2 *__r
 __global__ void __launch_bounds__(128)
 k_x_r2c(Dims d, FftPlan P, const double2 *__restrict__ roots, const double *__restrict__ phys,
         double2 *__restrict__ H, int RW, double nyq_scale) {
+    chain_begin();
     extern __shared__ double2 sm[];
     const int n = d.NX2;
     double2 *s_root = sm;
@@ -1441,6 +1456,7 @@ k_x_r2c(Dims d, FftPlan P, const double2 *__restrict__ roots, const double *__re
 __global__ void __launch_bounds__(256, 2)
 k_x_adjoint(Dims d, FftPlan P, const double2 *__restrict__ roots, const double2 *__restrict__ G,
             double2 *__restrict__ Lb, int RW) {
+    chain_begin();
     extern __shared__ double2 sm[];
     const int n = d.NX2;
     double2 *s_root = sm;
@@ -1708,8 +1724,7 @@ bool z_backward_r(const Dims &d, const double2 *roots, const C *F, C *G, int nf,
     dim3 grid((d.nkx + tl - 1) / tl, d.ny2, nf);
     return with_xsplit(d.NZ2, [&](auto a, auto b) {
         constexpr int N1 = decltype(a)::value, N2 = decltype(b)::value;
-        k_z_backward_r<N1, N2, C><<<grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(C)), s>>>(
-            d, roots, F, G, tl, coarse);
+        launch_chained(k_z_backward_r<N1, N2, C>, grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(C)), s, d, roots, F, G, tl, coarse);
     });
 }
 template <class C, bool MEAN>
@@ -1719,8 +1734,8 @@ bool x_cross_r(const Dims &d, const double2 *roots, const C *G, C *H, const doub
         const int per = 4 * kXHWarps;
         return with_xsplit(d.NX2, [&](auto a, auto b) {
             constexpr int N1 = decltype(a)::value, N2 = decltype(b)::value;
-            k_x_cross_h<N1, N2, C, MEAN><<<(unsigned)((rows + per - 1) / per), 32 * kXHWarps,
-                                           smem_xcross_h(N1, N2, sizeof(C)), s>>>(d, roots, G, H, mean);
+            launch_chained(k_x_cross_h<N1, N2, C, MEAN>, (unsigned)((rows + per - 1) / per), 32 * kXHWarps,
+                                           smem_xcross_h(N1, N2, sizeof(C)), s, d, roots, G, H, mean);
         });
     }
     const int rw = (d.xrw == 2 || d.xrw == 4) ? d.xrw : kRWr;   // even, at most kRWr
@@ -1731,13 +1746,11 @@ bool x_cross_r(const Dims &d, const double2 *roots, const C *G, C *H, const doub
             if (d.xrw == 3 || d.xrw == 5) {   // 4 or 2 rows, forward phases split over lane pairs
                 const int srw = d.xrw == 3 ? 4 : 2;
                 dim3 sgrid((d.NZ2 + srw - 1) / srw, d.ny2);
-                k_x_cross_r<N1, N2, C, MEAN, true><<<sgrid, 16 * 3 * srw, smem_xcross_r(N1, N2, sizeof(C), srw), s>>>(
-                    d, roots, G, H, srw, mean);
+                launch_chained(k_x_cross_r<N1, N2, C, MEAN, true>, sgrid, 16 * 3 * srw, smem_xcross_r(N1, N2, sizeof(C), srw), s, d, roots, G, H, srw, mean);
                 return;
             }
         }
-        k_x_cross_r<N1, N2, C, MEAN><<<grid, 16 * 3 * rw, smem_xcross_r(N1, N2, sizeof(C)), s>>>(
-            d, roots, G, H, rw, mean);
+        launch_chained(k_x_cross_r<N1, N2, C, MEAN>, grid, 16 * 3 * rw, smem_xcross_r(N1, N2, sizeof(C)), s, d, roots, G, H, rw, mean);
     });
 }
 template <class C>
@@ -1747,8 +1760,7 @@ bool z_forward_r(const Dims &d, const double2 *roots, const C *H, C *F, int nf, 
     dim3 grid((d.nkx + tl - 1) / tl, d.ny2, nf);
     return with_xsplit(d.NZ2, [&](auto a, auto b) {
         constexpr int N1 = decltype(a)::value, N2 = decltype(b)::value;
-        k_z_forward_r<N1, N2, C><<<grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(C)), s>>>(
-            d, roots, H, F, tl, coarse);
+        launch_chained(k_z_forward_r<N1, N2, C>, grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(C)), s, d, roots, H, F, tl, coarse);
     });
 }
 
@@ -1758,8 +1770,7 @@ bool launch_z_backward_peers(const Dims &d, const double2 *roots, const PeerCols
     dim3 grid((d.nkx + tl - 1) / tl, d.ny2, 6);
     return with_xsplit(d.NZ2, [&](auto a, auto b) {
         constexpr int N1 = decltype(a)::value, N2 = decltype(b)::value;
-        k_z_backward_peers<N1, N2><<<grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(double2)), s>>>(
-            d, roots, pc, G, tl);
+        launch_chained(k_z_backward_peers<N1, N2>, grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(double2)), s, d, roots, pc, G, tl);
     });
 }
 
@@ -1769,8 +1780,7 @@ bool launch_z_forward_peers(const Dims &d, const double2 *roots, const double2 *
     dim3 grid((d.nkx + tl - 1) / tl, d.ny2, 3);
     return with_xsplit(d.NZ2, [&](auto a, auto b) {
         constexpr int N1 = decltype(a)::value, N2 = decltype(b)::value;
-        k_z_forward_peers<N1, N2><<<grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(double2)), s>>>(
-            d, roots, H, pc, tl);
+        launch_chained(k_z_forward_peers<N1, N2>, grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(double2)), s, d, roots, H, pc, tl);
     });
 }
 
@@ -1780,7 +1790,7 @@ void launch_z_backward(const Dims &d, const FftPlan &P, const double2 *roots, co
     const int tl = z_lines(d);
     if (launch_z_any(d, roots, F, G, nf, true, tl, coarse, s)) return;
     dim3 grid((d.nkx + tl - 1) / tl, d.ny2, nf);
-    k_z_backward<<<grid, 256, smem_zfft(d), s>>>(d, P, roots, F, G, tl, coarse);
+    launch_chained(k_z_backward, grid, 256, smem_zfft(d), s, d, P, roots, F, G, tl, coarse);
 }
 
 void launch_x_cross(const Dims &d, const FftPlan &P, const double2 *roots, const double2 *G,
@@ -1788,7 +1798,7 @@ void launch_x_cross(const Dims &d, const FftPlan &P, const double2 *roots, const
     if (x_cross_r<double2, false>(d, roots, G, H, nullptr, s)) return;
     if (launch_x_cross_any(d, roots, G, H, s)) return;
     dim3 grid((d.NZ2 + kRW - 1) / kRW, d.ny2);
-    k_x_cross<<<grid, 256, smem_xcross(d), s>>>(d, P, roots, G, H, kRW);
+    launch_chained(k_x_cross, grid, 256, smem_xcross(d), s, d, P, roots, G, H, kRW);
 }
 
 void launch_z_forward(const Dims &d, const FftPlan &P, const double2 *roots, const double2 *H,
@@ -1797,7 +1807,7 @@ void launch_z_forward(const Dims &d, const FftPlan &P, const double2 *roots, con
     const int tl = z_lines(d);
     if (launch_z_any(d, roots, H, F, nf, false, tl, coarse, s)) return;
     dim3 grid((d.nkx + tl - 1) / tl, d.ny2, nf);
-    k_z_forward<<<grid, 256, smem_zfft(d), s>>>(d, P, roots, H, F, tl, coarse);
+    launch_chained(k_z_forward, grid, 256, smem_zfft(d), s, d, P, roots, H, F, tl, coarse);
 }
 
 // FP32 stage buffers (mixed precision): register forms only.
@@ -1817,11 +1827,11 @@ void launch_x_adjoint(const Dims &d, const FftPlan &P, const double2 *roots, con
     const bool reg = with_xsplit(d.NX2, [&](auto a, auto b) {
         constexpr int N1 = decltype(a)::value, N2 = decltype(b)::value;
         dim3 grid((d.NZ2 + kRWar - 1) / kRWar, d.ny2);
-        k_x_adjoint_r<N1, N2><<<grid, 16 * 5 * kRWar, smem_xadjoint_r(N1, N2), s>>>(d, roots, G, L, kRWar);
+        launch_chained(k_x_adjoint_r<N1, N2>, grid, 16 * 5 * kRWar, smem_xadjoint_r(N1, N2), s, d, roots, G, L, kRWar);
     });
     if (reg) return;
     dim3 grid((d.NZ2 + kRWa - 1) / kRWa, d.ny2);
-    k_x_adjoint<<<grid, 256, smem_xadjoint(d), s>>>(d, P, roots, G, L, kRWa);
+    launch_chained(k_x_adjoint, grid, 256, smem_xadjoint(d), s, d, P, roots, G, L, kRWa);
 }
 
 bool ydct_available(const Dims &d, const Tables &t) {
@@ -1839,9 +1849,9 @@ bool ydct(const Dims &d, const Tables &t, int nf, bool ana, const YdctArgs<CT> &
             constexpr int TL = decltype(w)::value;
             const size_t sm = smem_ydct(N1, N2, TL);
             if (ana)
-                k_ydct_r<N1, N2, true, TL, CT><<<grid, 16 * TL, sm, s>>>(d, t.root_y, t.cosy, A);
+                launch_chained(k_ydct_r<N1, N2, true, TL, CT>, grid, 16 * TL, sm, s, d, t.root_y, t.cosy, A);
             else
-                k_ydct_r<N1, N2, false, TL, CT><<<grid, 16 * TL, sm, s>>>(d, t.root_y, t.cosy, A);
+                launch_chained(k_ydct_r<N1, N2, false, TL, CT>, grid, 16 * TL, sm, s, d, t.root_y, t.cosy, A);
         });
     });
     return reg || launch_ydct_any(d, t, nf, ana, A, s);
@@ -1922,11 +1932,11 @@ void launch_x_moments(const Dims &d, const FftPlan &P, const double2 *roots, con
     const bool reg = with_xsplit(d.NX2, [&](auto a, auto b) {
         constexpr int N1 = decltype(a)::value, N2 = decltype(b)::value;
         const size_t sm = smem_xmoments_r(N1, N2);
-        if (nf == 5) k_x_moments_r<N1, N2, 3><<<grid, 16 * 12, sm, s>>>(d, roots, G, partial, phys);
-        else k_x_moments_r<N1, N2, 2><<<grid, 16 * 12, sm, s>>>(d, roots, G, partial, phys);
+        if (nf == 5) launch_chained(k_x_moments_r<N1, N2, 3>, grid, 16 * 12, sm, s, d, roots, G, partial, phys);
+        else launch_chained(k_x_moments_r<N1, N2, 2>, grid, 16 * 12, sm, s, d, roots, G, partial, phys);
     });
     if (reg) return;
-    k_x_moments<<<grid, 256, smem_xmoments(d), s>>>(d, P, roots, G, kRWm, partial, phys, nf);
+    launch_chained(k_x_moments, grid, 256, smem_xmoments(d), s, d, P, roots, G, kRWm, partial, phys, nf);
 }
 
 // The coarse grid doubles (c2r) / halves (r2c) a full-spectrum x Nyquist bin
@@ -1934,13 +1944,13 @@ void launch_x_moments(const Dims &d, const FftPlan &P, const double2 *roots, con
 void launch_x_c2r(const Dims &d, const FftPlan &P, const double2 *roots, const double2 *G,
                   double *phys, cudaStream_t s, bool coarse) {
     dim3 grid((d.NZ2 + kRWs - 1) / kRWs, d.ny2);
-    k_x_c2r<<<grid, 128, smem_xsingle(d), s>>>(d, P, roots, G, phys, kRWs, coarse ? 2.0 : 1.0);
+    launch_chained(k_x_c2r, grid, 128, smem_xsingle(d), s, d, P, roots, G, phys, kRWs, coarse ? 2.0 : 1.0);
 }
 
 void launch_x_r2c(const Dims &d, const FftPlan &P, const double2 *roots, const double *phys,
                   double2 *H, cudaStream_t s, bool coarse) {
     dim3 grid((d.NZ2 + kRWs - 1) / kRWs, d.ny2);
-    k_x_r2c<<<grid, 128, smem_xsingle(d), s>>>(d, P, roots, phys, H, kRWs, coarse ? 0.5 : 1.0);
+    launch_chained(k_x_r2c, grid, 128, smem_xsingle(d), s, d, P, roots, phys, H, kRWs, coarse ? 0.5 : 1.0);
 }
 
 }  // namespace cdns

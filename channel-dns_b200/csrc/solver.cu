@@ -294,6 +294,46 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
     }
     cp_async_commit();
 
+    // lane = 16 p + 2 cl + r: parity p, column cl of the block, part r (re, im)
+    const int p = lane >> 4, cl = (lane >> 1) & (TC - 1), r = lane & 1;
+    const int own = 2 * cl + r, oth = own ^ 1;
+    const int col = col0 + cl;
+    const bool live = col < ncol;
+    const int ccol = live ? col : ncol - 1;
+    const double ax = t.wavx[ccol % nkx], az = t.wavz[ccol / nkx];
+    const double sx = r ? ax : -ax, sz = r ? az : -az;
+    const bool zero_col = col == d.zc;
+    double *T = reinterpret_cast<double *>(tile);
+    const double *ad = s_ad + cl * AS;
+    bool pivot_fail = false;
+    // warps 1-3 hold the velocity pivots in registers while warp 0 solves the pressure
+    constexpr int kHoldCols = (TC + 2) / 3, kHoldRows = 8;   // NYS + 1 <= 256
+    double hold[kHoldCols][kHoldRows];
+    // warp 0's lanes fetch their column's influence data before the chains run:
+    // lane p uses sigma_0's entry p, and v of the first response at y = ny - p
+    const int coln = min(ccol / nkx, 2 * d.NZS - ccol / nkx) * nkx + ccol % nkx;   // the kz <= 0 column
+    double i00 = 0.0, i01 = 0.0, i10 = 0.0, i11 = 0.0, sg = 1.0, pn = 0.0, vn = 0.0, tail = 0.0;
+    double wt = 0.0, wb = 0.0, pt = 0.0, pb = 0.0, wp = 0.0;   // wall data of the pressure, its w
+    if (w == 0) {
+        const long long o_n = spectral_base(d, coln / nkx, coln % nkx) + (long long)ny * d.sy;
+        i00 = st.inf_div[coln].x;
+        i01 = st.inf_div[ncol + coln].x;
+        i10 = st.inf_div[2 * ncol + coln].x;
+        i11 = st.inf_div[3 * ncol + coln].x;
+        sg = st.sigma0[p * ncol + coln].x;
+        pn = st.p_inf[o_n];
+        vn = st.v_inf[d.Ns + o_n - p * d.sy];
+        wp = st.wn_p[ccol];
+        if (s.bc_p) {
+            wt = reinterpret_cast<const double *>(s.bc_p + ccol)[r];
+            wb = reinterpret_cast<const double *>(s.bc_p + ncol + ccol)[r];
+        } else {
+            wt = reinterpret_cast<const double *>(s.bw + ccol)[r];
+            wb = reinterpret_cast<const double *>(s.bw + ncol + ccol)[r];
+            pt = reinterpret_cast<const double *>(s.B_prev + ccol)[r];
+            pb = reinterpret_cast<const double *>(s.B_prev + ncol + ccol)[r];
+        }
+    }
     // ---- stage R = a0 u + a1 u_prev + b0 N + b1 N_prev; sums of N_y --------
     // (the loads of two rows are issued before the first use)
     {
@@ -332,25 +372,6 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
     __syncthreads();
 
     // ---- chains ------------------------------------------------------------
-    // lane = 16 p + 2 cl + r: parity p, column cl of the block, part r (re, im)
-    const int p = lane >> 4, cl = (lane >> 1) & (TC - 1), r = lane & 1;
-    const int own = 2 * cl + r, oth = own ^ 1;
-    const int col = col0 + cl;
-    const bool live = col < ncol;
-    const int ccol = live ? col : ncol - 1;
-    const double ax = t.wavx[ccol % nkx], az = t.wavz[ccol / nkx];
-    const double sx = r ? ax : -ax, sz = r ? az : -az;
-    const bool zero_col = col == d.zc;
-    double *T = reinterpret_cast<double *>(tile);
-    const double *ad = s_ad + cl * AS;
-    bool pivot_fail = false;
-    // warps 1-3 hold the velocity pivots in registers while warp 0 solves the pressure
-    constexpr int kHoldCols = (TC + 2) / 3, kHoldRows = 8;   // NYS + 1 <= 256
-    double hold[kHoldCols][kHoldRows];
-    // warp 0's lanes fetch their column's influence data before the chains run:
-    // lane p uses sigma_0's entry p, and v of the first response at y = ny - p
-    const int coln = min(ccol / nkx, 2 * d.NZS - ccol / nkx) * nkx + ccol % nkx;   // the kz <= 0 column
-    double i00 = 0.0, i01 = 0.0, i10 = 0.0, i11 = 0.0, sg = 1.0, pn = 0.0, vn = 0.0, tail = 0.0;
     if (w == 0) {
         const double *sum = T + 6 * S;
         double lower, upper;
@@ -361,32 +382,22 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
         const double other = __shfl_xor_sync(kFull, mine, 16);
         const double even = p ? other : mine, odd = p ? mine : other;
         if (s.bc_p) {
-            lower = reinterpret_cast<const double *>(s.bc_p + ccol)[r];
-            upper = reinterpret_cast<const double *>(s.bc_p + ncol + ccol)[r];
+            lower = wt;
+            upper = wb;
         } else {
             // pressure wall data (src/solver/eqsolve_pv.cpp:322-337) and its
             // combination b0 B + b1 B_prev (src/sim/simulation.cpp:146-150)
-            const double bt = reinterpret_cast<const double *>(s.bw + ccol)[r] + (even + odd);
-            const double bb = reinterpret_cast<const double *>(s.bw + ncol + ccol)[r] + (odd - even);
-            lower = s.b0 * bt + s.b1 * reinterpret_cast<const double *>(s.B_prev + ccol)[r];
-            upper = s.b0 * bb + s.b1 * reinterpret_cast<const double *>(s.B_prev + ncol + ccol)[r];
+            const double bt = wt + (even + odd);
+            const double bb = wb + (odd - even);
+            lower = s.b0 * bt + s.b1 * pt;
+            upper = s.b0 * bb + s.b1 * pb;
             if (live) reinterpret_cast<double *>(s.B_new + p * ncol + col)[r] = p ? bb : bt;
         }
         tail = T[(2 * S) + (ny - p) * (2 * TC) + own];   // R_1 at ny, ny - 1
-        {
-            const long long o_n = spectral_base(d, coln / nkx, coln % nkx) + (long long)ny * d.sy;
-            i00 = st.inf_div[coln].x;
-            i01 = st.inf_div[ncol + coln].x;
-            i10 = st.inf_div[2 * ncol + coln].x;
-            i11 = st.inf_div[3 * ncol + coln].x;
-            sg = st.sigma0[p * ncol + coln].x;
-            pn = st.p_inf[o_n];
-            vn = st.v_inf[d.Ns + o_n - p * d.sy];
-        }
         __syncwarp();   // the sums were read by every lane before P's sweep overwrites them
         DivergenceRhs rhs{T + oth, T + 2 * S + own, T + 4 * S + oth, sx, sz, ny};
         pivot_fail |= !tau_chain(ny, p, A.p_a, A.p_b, pp.G_pre == 0.0 && A.p_a == 0.0 && zero_col, lower, upper,
-                                 st.wn_p[ccol], s_w, t.WD, ad, T + 6 * S + own, rhs, [](double, double) {});
+                                 wp, s_w, t.WD, ad, T + 6 * S + own, rhs, [](double, double) {});
     } else {
 #pragma unroll
         for (int i = 0; i < kHoldCols; ++i) {

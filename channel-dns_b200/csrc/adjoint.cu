@@ -49,7 +49,7 @@ template <int E> __device__ __forceinline__ void deriv_T(int ny, const double2 (
     }
 }
 
-// Transpose of tau_warp (solver.cu): given the adjoint lz of the tau
+// Transpose of the tau solve (tau_chain, solver.cu): given the adjoint lz of the tau
 // solution, the adjoints of its right-hand side (lr) and of its wall data.
 template <int E>
 __device__ void tau_adj(int ny, double g, double a, double b, bool zero_col, double w, const double2 (&lz)[E],

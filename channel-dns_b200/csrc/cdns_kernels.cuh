@@ -95,7 +95,7 @@ bool launch_ydct_adjoint_synthesis(const Dims &d, const Tables &t, const double2
 // Output reduction, x stage on the coarse grid (Dims of the coarse grid):
 // c2r of G[nf] (u, v, w, p and, if nf = 5, div), per-point moments summed per
 // block into partial[NY+1][moment_blocks][22]; phys (may be null) receives u, v, w, p.
-int moment_blocks(const Dims &d, int nf);
+int moment_blocks(const Dims &d);
 void launch_x_moments(const Dims &d, const FftPlan &P, const double2 *roots, const double2 *G, double *partial,
                       double *phys, int nf, cudaStream_t s);
 // Transpose of x_cross about the forward fields G[6]: L[0..2] = lH in, L[0..5] = lG out.

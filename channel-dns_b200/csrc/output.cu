@@ -237,7 +237,7 @@ int ensure_output(cdns_ctx *c, bool snapshot) {
             (r = oalloc(c, w, ryd, ry.size())) ||
             (r = oalloc(c, w, w->pd, 2 * Ns)) || (r = oalloc(c, w, w->F, 5 * ny1 * d.ncol)) ||
             (r = oalloc(c, w, w->G, 5 * ny1 * dc.NZ2 * d.nkx)) ||
-            (r = oalloc(c, w, w->partial, ny1 * moment_blocks(dc, 5) * 22)) ||
+            (r = oalloc(c, w, w->partial, ny1 * moment_blocks(dc) * 22)) ||
             (r = oalloc(c, w, w->planes, ny1 * 22)) || (r = oalloc(c, w, w->flag, 1)))
             return r;
         CK(cudaMemcpyAsync(cy, cosy.data(), cosy.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
@@ -327,7 +327,7 @@ int enqueue_reduction(cdns_ctx *c, bool snapshot, bool check, bool sample = fals
     const int nf = check ? 5 : 4;
     launch_z_backward(dc, w->pz, w->tc.root_z, w->F, w->G, nf, s, true);
     launch_x_moments(dc, w->px, w->tc.root_x, w->G, w->partial, snapshot ? w->phys : nullptr, nf, s);
-    k_plane_finalize<<<dc.ny2, 192, 0, s>>>(moment_blocks(dc, nf), w->partial, w->planes, dc.ny2,
+    k_plane_finalize<<<dc.ny2, 192, 0, s>>>(moment_blocks(dc), w->partial, w->planes, dc.ny2,
                                             1.0 / ((double)dc.NX2 * (double)dc.NZ2), w->count, c->dpdx,
                                             sample ? w->stats : nullptr);
     CK(cudaGetLastError());

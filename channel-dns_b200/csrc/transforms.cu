@@ -1163,8 +1163,7 @@ k_x_adjoint_r(Dims d, const double2 *__restrict__ roots, const double2 *__restri
 // doubled (the coarse c2r convention).
 // ---------------------------------------------------------------------------
 constexpr int kMomentSlots = 22;
-// rows per block of k_x_moments_r: 12 lines
-__host__ __device__ constexpr int moment_rows(int lpr) { return 12 / lpr; }
+constexpr int kRWm = 4;           // rows per block of k_x_moments and k_x_moments_r
 constexpr int kMomentLanes = 8;   // threads that sum one slot (22 x 8 <= the block's threads)
 
 struct MomentAcc {
@@ -1210,13 +1209,16 @@ struct MomentAcc {
     }
 };
 
-// LPR lines per row: 3 with the divergence (nf = 5), 2 without; 12 / LPR rows per block.
+// LPR lines per row: 3 with the divergence (nf = 5), 2 without.  The rows and the
+// threads of a block are the same for both (a third of the threads has no line where
+// LPR = 2), so that a sample adds its points in the order of a check step: the
+// low-order bits of sums that cancel are then the same.
 template <int N1, int N2, int LPR>
 __global__ void __launch_bounds__(16 * 12)
 k_x_moments_r(Dims d, const double2 *__restrict__ roots, const double2 *__restrict__ G,
               double *__restrict__ partial, double *__restrict__ phys) {
     chain_begin();
-    constexpr int RW = moment_rows(LPR), nf = LPR == 3 ? 5 : 4;
+    constexpr int RW = kRWm, nf = LPR == 3 ? 5 : 4;
     using C = double2;
     constexpr int n = N1 * N2;
     constexpr int SP = N2 + 1;
@@ -1619,7 +1621,6 @@ template <typename Fn> bool with_xsplit(int nx2, Fn &&fn) {
     }
 }
 
-constexpr int kRWm = 4;    // rows per block of the output-reduction x stage
 size_t smem_xmoments_r(int n1, int n2) {
     const size_t L = 3 * kRWm;
     const size_t s1 = L * n1 * (n2 + 1), s2 = L * n1 * n2;
@@ -1919,16 +1920,12 @@ bool launch_ydct_analysis_fp32(const Dims &d, const Tables &t, const float2 *F, 
     return ydct(d, t, nf, true, A, s);
 }
 
-// x-stage blocks per plane of the output reduction for nf fields
-int moment_blocks(const Dims &d, int nf) {
-    const bool reg = with_xsplit(d.NX2, [](auto, auto) {});
-    const int rw = reg ? moment_rows(nf == 5 ? 3 : 2) : kRWm;
-    return (d.NZ2 + rw - 1) / rw;
-}
+// x-stage blocks per plane of the output reduction
+int moment_blocks(const Dims &d) { return (d.NZ2 + kRWm - 1) / kRWm; }
 
 void launch_x_moments(const Dims &d, const FftPlan &P, const double2 *roots, const double2 *G, double *partial,
                       double *phys, int nf, cudaStream_t s) {
-    dim3 grid(moment_blocks(d, nf), d.ny2);
+    dim3 grid(moment_blocks(d), d.ny2);
     const bool reg = with_xsplit(d.NX2, [&](auto a, auto b) {
         constexpr int N1 = decltype(a)::value, N2 = decltype(b)::value;
         const size_t sm = smem_xmoments_r(N1, N2);

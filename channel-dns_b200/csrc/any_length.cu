@@ -1,5 +1,5 @@
 // Register-form transforms of the product lengths without a compiled split of
-// their own (FP64 z and x stages, Chebyshev DCT): n = N1 x N2 with both factors
+// their own (z and x stages and Chebyshev DCT, FP64): n = N1 x N2 with both factors
 // among the in-register DFT lengths (reg_fft.cuh), chosen on the host and
 // switched over inside the kernels, so that one kernel serves every such length.
 //
@@ -308,10 +308,10 @@ constexpr int kYThreads = 256;
 __host__ __device__ constexpr int y_blocks(int maxr) { return maxr > 16 ? 2 : 3; }
 constexpr int kYPairs = 4;     // pairs of rows of a thread in flight
 constexpr int kYChunk = 13;    // (N/2 + 1) / R, rounded up, is at most this for N1, N2 <= 25
-template <int MAXR, bool ANA, class CT>
+template <int MAXR, bool ANA>
 __global__ void __launch_bounds__(kYThreads, y_blocks(MAXR))
 k_ydct_any(Dims d, int N1, int N2, int TL, int R, const double2 *__restrict__ roots,
-           const double *__restrict__ cosy, YdctArgs<CT> A) {
+           const double *__restrict__ cosy, YdctArgs<double2> A) {
     chain_begin();
     const int N = N1 * N2;
     const int KS = fft2_kstride(N2, TL);
@@ -335,7 +335,7 @@ k_ydct_any(Dims d, int N1, int N2, int TL, int R, const double2 *__restrict__ ro
     double2 y1 = mk(0.0, 0.0);
     {
         const double2 *S = nullptr;
-        const CT *F = nullptr;
+        const double2 *F = nullptr;
         if (!ANA) S = (f < A.nsplit ? A.spec0 + (long long)f * d.Ns : A.spec1 + (long long)(f - A.nsplit) * d.Ns) +
                       spectral_base(d, kzi, kx);
         else F = A.Fin + (long long)f * d.ny2 * d.fcol + (long long)kzi * nkx + kx;
@@ -349,8 +349,8 @@ k_ydct_any(Dims d, int N1, int N2, int TL, int R, const double2 *__restrict__ ro
                     xa[i] = (in && n < ncy) ? S[(long long)n * d.sy] : mk(0.0, 0.0);
                     xb[i] = (in && m < ncy) ? S[(long long)m * d.sy] : mk(0.0, 0.0);
                 } else {
-                    xa[i] = in ? cto<double2>(F[(long long)n * d.fcol]) : mk(0.0, 0.0);
-                    xb[i] = in ? cto<double2>(F[(long long)m * d.fcol]) : mk(0.0, 0.0);
+                    xa[i] = in ? F[(long long)n * d.fcol] : mk(0.0, 0.0);
+                    xb[i] = in ? F[(long long)m * d.fcol] : mk(0.0, 0.0);
                 }
             }
 #pragma unroll
@@ -407,20 +407,14 @@ k_ydct_any(Dims d, int N1, int N2, int TL, int R, const double2 *__restrict__ ro
         const int q = byN1(k);
         return Y[(k - q * N1) * KS + q * TL + l];
     };
-    CT *Fo = nullptr;
+    double2 *Fo = nullptr;
     double2 *So = nullptr;
     if (!ANA) Fo = A.Fout + (long long)f * d.ny2 * d.fcol + (long long)kzi * nkx + kx;
     else So = A.S + (long long)f * d.Ns + spectral_base(d, kzi, kx);
-    const bool to_mean = !ANA && A.mean && kzi == d.NZS && kx == 0;
     auto out = [&](int j, double2 v) {
         if (!lok) return;
         if (!ANA) {
-            if (to_mean) {
-                A.mean[f * d.ny2 + j] = v.x;
-                Fo[(long long)j * d.fcol] = mkc<CT>(0.0, 0.0);
-            } else {
-                Fo[(long long)j * d.fcol] = cto<CT>(cscale(j == 0 || j == N ? A.outE : A.outI, v));
-            }
+            Fo[(long long)j * d.fcol] = cscale(j == 0 || j == N ? A.outE : A.outI, v);
         } else if (j < ncy) {
             So[(long long)j * d.sy] = cscale(j == 0 ? A.s0 : A.sk, v);
         }
@@ -541,10 +535,8 @@ cudaError_t configure_any_kernels(const Dims &d) {
         const size_t sm = smem_y(a, b, y_lines(d, a, b));
         with_instance(a, b, [&](auto r) {
             constexpr int M = decltype(r)::value;
-            up(k_ydct_any<M, false, double2>, sm);
-            up(k_ydct_any<M, true, double2>, sm);
-            up(k_ydct_any<M, false, float2>, sm);
-            up(k_ydct_any<M, true, float2>, sm);
+            up(k_ydct_any<M, false>, sm);
+            up(k_ydct_any<M, true>, sm);
         });
     }
     return e;
@@ -576,8 +568,7 @@ bool launch_x_cross_any(const Dims &d, const double2 *roots, const double2 *G, d
     return true;
 }
 
-template <class CT>
-bool launch_ydct_any(const Dims &d, const Tables &t, int nf, bool ana, const YdctArgs<CT> &A, cudaStream_t s) {
+bool launch_ydct_any(const Dims &d, const Tables &t, int nf, bool ana, const YdctArgs<double2> &A, cudaStream_t s) {
     int a, b;
     if (d.NY2 % 2 || !any_split(d.NY2, a, b)) return false;
     const int R = y_rows(a, b), tl = y_lines(d, a, b);
@@ -585,12 +576,10 @@ bool launch_ydct_any(const Dims &d, const Tables &t, int nf, bool ana, const Ydc
     const size_t sm = smem_y(a, b, tl);
     with_instance(a, b, [&](auto r) {
         constexpr int M = decltype(r)::value;
-        if (ana) launch_chained(k_ydct_any<M, true, CT>, grid, R * tl, sm, s, d, a, b, tl, R, t.root_y, t.cosy, A);
-        else launch_chained(k_ydct_any<M, false, CT>, grid, R * tl, sm, s, d, a, b, tl, R, t.root_y, t.cosy, A);
+        if (ana) launch_chained(k_ydct_any<M, true>, grid, R * tl, sm, s, d, a, b, tl, R, t.root_y, t.cosy, A);
+        else launch_chained(k_ydct_any<M, false>, grid, R * tl, sm, s, d, a, b, tl, R, t.root_y, t.cosy, A);
     });
     return true;
 }
-template bool launch_ydct_any<double2>(const Dims &, const Tables &, int, bool, const YdctArgs<double2> &, cudaStream_t);
-template bool launch_ydct_any<float2>(const Dims &, const Tables &, int, bool, const YdctArgs<float2> &, cudaStream_t);
 
 }  // namespace cdns

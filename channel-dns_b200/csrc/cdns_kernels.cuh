@@ -76,7 +76,8 @@ bool launch_z_forward_peers(const Dims &ds, const double2 *roots, const double2 
 // Chebyshev synthesis (ana = false: spectral src0/src1 as in launch_ysynth ->
 // F) or analysis (ana = true: F in src0 -> spectral) in the FFT (DCT-I) form;
 // false if NY2 has no register split (the caller takes the matrix form).
-bool ydct_available(const Dims &d, const Tables &t);
+// (fp32: for FP32 stage buffers, which take the compiled splits alone)
+bool ydct_available(const Dims &d, const Tables &t, bool fp32 = false);
 bool launch_ydct(const Dims &d, const Tables &t, const double2 *src0, const double2 *src1, int nsplit, int nf,
                  double2 *out, bool ana, cudaStream_t s);
 // The same for FP32 stage buffers: the synthesis keeps the (kz, kx) = (0, 0)
@@ -151,6 +152,7 @@ struct StepArgs {
     double a0, a1, b0, b1;
     const double2 *bc_p;        // if set: pressure wall data [2][ncol] used as is
     int solve_only;             // 1: solve_modes alone (no zero-mode / flow correction)
+    int scan;                   // 1: by warp scans (solver_scan.cu), om and bw_out not used
     double2 *om;                // if set: the curl of u_out [3][Ns] and its pressure-wall sums
     double2 *bw_out;            // [2][ncol]
 };
@@ -164,6 +166,10 @@ void setup_solver(const Dims &d, const Tables &t, const PhysParams &pp, double g
 void launch_step_solve(const Dims &d, const Tables &t, const PhysParams &pp, double g_v,
                        const SolverState &st, const StepArgs &a, cudaStream_t s);
 cudaError_t configure_solver_kernels(const Dims &d);
+// ---- solver_scan.cu ---- (launch_step_solve with a.scan)
+void launch_scan_solve(const Dims &d, const Tables &t, const PhysParams &pp, double g_v, const SolverState &st,
+                       const StepArgs &a, cudaStream_t s);
+cudaError_t configure_scan_solve(const Dims &d);
 // Pressure wall data of a standalone nonlinear evaluation: B = bw + endpoint sums of N_y.
 void launch_pressure_bc(const Dims &d, const double2 *N, const double2 *bw, double2 *B,
                         cudaStream_t s);

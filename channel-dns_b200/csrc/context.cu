@@ -89,6 +89,11 @@ void ensure_curl(cdns_ctx *c) {
     c->om_current = true;
 }
 
+void prepare_step(cdns_ctx *c) {
+    if (c->mixed) c->om_current = false;
+    else ensure_curl(c);
+}
+
 void enqueue_nonlinear(cdns_ctx *c, const double2 *u, double2 *N, bool prof, int step_slot, double2 *G_fp64) {
     const Dims &d = c->d;
     cudaStream_t s = c->stream;
@@ -155,10 +160,14 @@ void enqueue_solve(cdns_ctx *c, double a0, double a1, double b0, double b1, doub
     a.a1 = a1;
     a.b0 = b0;
     a.b1 = b1;
-    a.om = c->om;
-    a.bw_out = c->bwb[1 - k];
+    if (c->mixed) {
+        a.scan = 1;
+    } else {
+        a.om = c->om;
+        a.bw_out = c->bwb[1 - k];
+    }
     launch_step_solve(c->d, c->t, c->pp, g_v, c->st, a, c->stream);
-    c->om_current = true;   // of u_out, the current velocity once the caller rotates
+    c->om_current = !c->mixed;   // of u_out, the current velocity once the caller rotates
 }
 
 int require_whole(const cdns_ctx *c) {
@@ -201,7 +210,7 @@ int one_step(cdns_ctx *c, int it) {
         int r = do_setup(c, g);
         if (r) return r;
     }
-    ensure_curl(c);
+    prepare_step(c);
     if (c->prof) {
         if (c->prof_steps >= kMaxProfSteps) return fail(CDNS_ERR_STATE, "profiling window full");
         enqueue_step_body(c, a0, a1, b0, b1, g, true, c->prof_steps);
@@ -675,6 +684,7 @@ int cdns_solve(cdns_ctx *c, double g, const double *rhs, const double *pbc, cons
     a.err = c->err;
     a.a0 = 1.0;
     a.solve_only = 1;
+    a.scan = c->mixed;
     launch_step_solve(d, c->t, c->pp, g, c->st, a, c->stream);
     launch_interleave(d, c->aux2, c->aux, 3, c->stream);
     launch_interleave(d, c->F, c->H, 1, c->stream);
@@ -873,7 +883,7 @@ int batch_step(cdns_batch *b, int it) {
         }
         return CDNS_OK;
     }
-    for (cdns_ctx *m : b->members) ensure_curl(m);
+    for (cdns_ctx *m : b->members) prepare_step(m);
     cudaGraphExec_t &ge = b->graph[b->members[0]->cur];
     if (!ge) {
         cudaGraph_t graph;

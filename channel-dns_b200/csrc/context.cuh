@@ -66,7 +66,7 @@ struct cdns_ctx {
     double2 *bw = nullptr;                // ... of the last nonlinear evaluation (one of the two)
     double2 *F = nullptr, *G = nullptr, *H = nullptr, *aux = nullptr, *aux2 = nullptr, *zero3 = nullptr;
     double2 *om = nullptr;                // vorticity of the velocity being transformed
-    bool om_current = false;              // om and bwb[cur] belong to U[cur] (the solve leaves them so)
+    bool om_current = false;              // om and bwb[cur] belong to U[cur] (the FP64 solve leaves them so)
     bool mixed = false;                   // FP32 fine-grid stages (CDNS_PRECISION_MIXED)
     double *mean = nullptr;               // mixed: FP64 (kz, kx) = (0, 0) profiles [6][NY2+1]
     double *phys = nullptr;
@@ -116,6 +116,9 @@ void step_coefficients(int it, double dt, double re, double &a0, double &a1, dou
 // om and bwb[cur] of the current velocity: the last solve left them, unless the
 // velocity or om changed since.  Called before a step is enqueued or replayed.
 void ensure_curl(cdns_ctx *c);
+// Before a step is enqueued, captured or replayed: ensure_curl where the solve leaves
+// the curl for the next step (FP64); a mixed step launches its own, also inside a graph.
+void prepare_step(cdns_ctx *c);
 // Nonlinear stages u -> N (planar spectral) and bw; G_fp64 (FP64 contexts)
 // receives the z-physical fields of u and omega, c->G if null.
 void enqueue_nonlinear(cdns_ctx *c, const double2 *u, double2 *N, bool prof, int step_slot,

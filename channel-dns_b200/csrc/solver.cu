@@ -702,12 +702,14 @@ void launch_pressure_bc(const Dims &d, const double2 *N, const double2 *bw, doub
 cudaError_t configure_solver_kernels(const Dims &d) {
     cudaError_t e = configure_setup_kernels(d);
     if (e != cudaSuccess) return e;
-    if (lane_elems(d) == 0) return cudaErrorInvalidValue;   // more than 256 Chebyshev coefficients
+    e = configure_scan_solve(d);   // (refuses more than 256 Chebyshev coefficients)
+    if (e != cudaSuccess) return e;
     return raise_smem(k_solve, solve_smem(d));
 }
 
 void launch_step_solve(const Dims &d, const Tables &t, const PhysParams &pp, double g_v,
                        const SolverState &st, const StepArgs &a, cudaStream_t s) {
+    if (a.scan) return launch_scan_solve(d, t, pp, g_v, st, a, s);
     SolveArgs A{};
     A.p_a = pp.a_pre0;
     A.p_b = pp.b_pre0;

@@ -112,7 +112,6 @@ cudaError_t configure_any_kernels(const Dims &d);
 bool launch_z_any(const Dims &d, const double2 *roots, const double2 *in, double2 *out, int nf, bool backward,
                   int lines, bool coarse, cudaStream_t s);
 bool launch_x_cross_any(const Dims &d, const double2 *roots, const double2 *G, double2 *H, cudaStream_t s);
-template <class CT>
-bool launch_ydct_any(const Dims &d, const Tables &t, int nf, bool ana, const YdctArgs<CT> &A, cudaStream_t s);
+bool launch_ydct_any(const Dims &d, const Tables &t, int nf, bool ana, const YdctArgs<double2> &A, cudaStream_t s);
 
 }  // namespace cdns

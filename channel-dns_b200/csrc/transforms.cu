@@ -252,6 +252,8 @@ __host__ __device__ constexpr size_t ydct_slots(int n1, int n2, int tl) {
 // (21 at TL = 13, whose blocks take 7 warps).  Left free, TL = 11 took 86 and 3
 // blocks: the synthesis ran in 97 instead of 87 us at Re_tau180.
 __host__ __device__ constexpr int ydct_blocks(int tl) { return tl == 8 ? 6 : tl == 11 ? 4 : 3; }
+// s v with its own rounding (never contracted into a following addition)
+__device__ __forceinline__ double2 cscale_rn(double s, double2 v) { return mk(__dmul_rn(s, v.x), __dmul_rn(s, v.y)); }
 template <int N1, int N2, bool ANA, int TL, class CT>
 __global__ void __launch_bounds__(16 * TL, ydct_blocks(TL))
 k_ydct_r(Dims d, const double2 *__restrict__ roots, const double *__restrict__ cosy, YdctArgs<CT> A) {
@@ -276,9 +278,17 @@ k_ydct_r(Dims d, const double2 *__restrict__ roots, const double *__restrict__ c
     // ---- y_n, y_{N-n} from x_n, x_{N-n}; partials of Y_1 = (x_0 - x_N)/2 +
     // sum_{n=1}^{N-1} x_n cos(pi n / N); all loads are issued before the first use
     constexpr int NI = N / 2 / R + 1;
+    // FP32 stages (ROWS): a thread's partial runs over its rows r, r + R, ... < N one
+    // after the other, those above N/2 loaded again, instead of over its pairs; row N - n
+    // takes its own table entry, and the products by it are rounded before they are added.
+    // So their results keep their bits (why it matters: solver_scan.cu).
+    constexpr bool ROWS = sizeof(CT) == 8;
+    constexpr int NC = ROWS ? (N - 1) / R - N / 2 / R + 1 : 1;
     double2 xa[NI], xb[NI];
+    const double2 *S = nullptr;
+    const CT *F = nullptr;
     if (!ANA) {
-        const double2 *S = (f < A.nsplit ? A.spec0 + (long long)f * d.Ns : A.spec1 + (long long)(f - A.nsplit) * d.Ns) +
+        S = (f < A.nsplit ? A.spec0 + (long long)f * d.Ns : A.spec1 + (long long)(f - A.nsplit) * d.Ns) +
                            spectral_base(d, kzi, kx);
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
@@ -287,7 +297,7 @@ k_ydct_r(Dims d, const double2 *__restrict__ roots, const double *__restrict__ c
             xb[i] = (n <= N / 2 && m < ncy && lok) ? S[(long long)m * d.sy] : mk(0.0, 0.0);
         }
     } else {
-        const CT *F = A.Fin + (long long)f * d.ny2 * d.fcol + (long long)kzi * nkx + kx;
+        F = A.Fin + (long long)f * d.ny2 * d.fcol + (long long)kzi * nkx + kx;
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
             const int n = r + R * i, m = N - n;
@@ -295,7 +305,7 @@ k_ydct_r(Dims d, const double2 *__restrict__ roots, const double *__restrict__ c
             xb[i] = (n <= N / 2 && lok) ? cto<double2>(F[(long long)m * d.fcol]) : mk(0.0, 0.0);
         }
     }
-    double2 y1 = mk(0.0, 0.0);
+    double2 y1 = mk(0.0, 0.0), ends = mk(0.0, 0.0);
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
         const int n = r + R * i;
@@ -306,14 +316,37 @@ k_ydct_r(Dims d, const double2 *__restrict__ roots, const double *__restrict__ c
         const double2 a = cscale(w0, xa[i]), b = cscale(w1, xb[i]);
         const double2 h = cscale(0.5, cadd(a, b)), df = csub(a, b);
         const double sn = cosy[n < N / 2 ? n + (3 * N) / 2 : 0];   // sin(pi n / N)
-        y1 = cadd(y1, cscale(n == 0 ? 0.5 : cosy[n], df));   // cos(pi (N - n) / N) = -cos(pi n / N)
-        Y[row(n)] = csub(h, cscale(sn, df));
-        if (n > 0 && n < N / 2) Y[row(N - n)] = cadd(h, cscale(sn, df));
+        if (!ROWS) y1 = cadd(y1, cscale(n == 0 ? 0.5 : cosy[n], df));   // cos(pi (N - n) / N) = -cos(pi n / N)
+        else if (n == 0) ends = cscale(0.5, df);
+        else y1 = cadd(y1, cscale(cosy[n], a));
+        if (!ROWS) {
+            Y[row(n)] = csub(h, cscale(sn, df));
+            if (n > 0 && n < N / 2) Y[row(N - n)] = cadd(h, cscale(sn, df));
+        } else {
+            Y[row(n)] = csub(h, cscale_rn(sn, df));
+            if (n > 0 && n < N / 2) Y[row(N - n)] = cadd(h, cscale_rn(cosy[N / 2 - n], df));
+        }
+    }
+    if (ROWS) {
+        const double w = !ANA ? A.in1 : A.inI;
+        double2 x[NC];
+#pragma unroll
+        for (int i = 0; i < NC; ++i) {
+            const int n = r + R * (N / 2 / R + i);
+            const bool in = n > N / 2 && n < N && lok;
+            if (!ANA) x[i] = in && n < ncy ? S[(long long)n * d.sy] : mk(0.0, 0.0);
+            else x[i] = in ? cto<double2>(F[(long long)n * d.fcol]) : mk(0.0, 0.0);
+        }
+#pragma unroll
+        for (int i = 0; i < NC; ++i) {
+            const int n = r + R * (N / 2 / R + i);
+            if (n > N / 2 && n < N) y1 = cadd(y1, cscale(cosy[n], cscale(w, x[i])));
+        }
     }
     P[r * TL + l] = y1;
     __syncthreads();
     if (r == 0) {
-        double2 acc = P[l];
+        double2 acc = ROWS ? cadd(ends, P[l]) : P[l];
 #pragma unroll
         for (int q = 1; q < R; ++q) acc = cadd(acc, P[q * TL + l]);
         Y1[l] = acc;
@@ -1835,13 +1868,13 @@ void launch_x_adjoint(const Dims &d, const FftPlan &P, const double2 *roots, con
     launch_chained(k_x_adjoint, grid, 256, smem_xadjoint(d), s, d, P, roots, G, L, kRWa);
 }
 
-bool ydct_available(const Dims &d, const Tables &t) {
-    return t.root_y && d.NY2 % 2 == 0 && (with_xsplit(d.NY2, [](auto, auto) {}) || any_length(d.NY2));
+bool ydct_available(const Dims &d, const Tables &t, bool fp32) {
+    return t.root_y && d.NY2 % 2 == 0 && (with_xsplit(d.NY2, [](auto, auto) {}) || (!fp32 && any_length(d.NY2)));
 }
 
 template <class CT>
 bool ydct(const Dims &d, const Tables &t, int nf, bool ana, const YdctArgs<CT> &A, cudaStream_t s) {
-    if (!ydct_available(d, t)) return false;
+    if (!ydct_available(d, t, sizeof(CT) == 8)) return false;
     const int tl = ydct_lines(d);
     dim3 grid((d.nkx + tl - 1) / tl, d.nkz, nf);
     const bool reg = with_xsplit(d.NY2, [&](auto a, auto b) {
@@ -1855,7 +1888,8 @@ bool ydct(const Dims &d, const Tables &t, int nf, bool ana, const YdctArgs<CT> &
                 launch_chained(k_ydct_r<N1, N2, false, TL, CT>, grid, 16 * TL, sm, s, d, t.root_y, t.cosy, A);
         });
     });
-    return reg || launch_ydct_any(d, t, nf, ana, A, s);
+    if constexpr (sizeof(CT) == 16) return reg || launch_ydct_any(d, t, nf, ana, A, s);
+    else return reg;
 }
 bool launch_ydct(const Dims &d, const Tables &t, const double2 *src0, const double2 *src1, int nsplit, int nf,
                  double2 *out, bool ana, cudaStream_t s) {

@@ -95,7 +95,7 @@ int measure_fp32(cdns_ctx *c, Choice &out) {
             }
         }
     }
-    if (!ydct_available(d, c->t)) return CDNS_OK;
+    if (!ydct_available(d, c->t, true)) return CDNS_OK;
     float2 *F = reinterpret_cast<float2 *>(c->F);
     Tables t = c->t;
     float m_syn, f_syn, m_ana, f_ana;

@@ -30,7 +30,7 @@
 // us; a warp per column with shuffle scans, twelve fields and a curl kernel of its
 // own took 176 + 32 us.
 #include "cdns_kernels.cuh"
-#include "warp_columns.cuh"
+#include "tau_warp.cuh"
 
 namespace cdns {
 
@@ -257,8 +257,71 @@ template <int C> struct VelocityRhs {
     }
 };
 
+// The real parts of u and w of the (kz, kx) = (0, 0) column before their pressure
+// gradient, by warp scans and from the multistep state: the column whose fluxes give
+// dp/dx and dp/dz where the flow rate is fixed.  dp/dx = (Q - q) / q_unit, with Q - q
+// some 4e-6 of Q, shows each last bit of this column as 5e-11, so that the order of its
+// operations is part of the result: by the chains, dp/dx of a 32 x 49 x 32 channel is
+// 5e-11 to 1e-10 off after six steps.  No pressure enters (kx = kz = 0), nor do the
+// corrections.  Warp 3 of one block does it beside the pressure chains: a step of 32 x
+// 33 x 32 takes 36.9 us with it and without (41.0 with u and w one after the other
+// beside the velocity chains).  (u, w) are one double2 column where their wall conditions
+// are the same (c = 0, both), else one after the other.
+template <int E>
+__device__ __noinline__ void flux_column(const Dims &d, const Tables &t, const PhysParams &pp, double g,
+                                         const SolverState &st, const StepArgs &s, double2 *v_out, int c, bool both) {
+    const int ny = d.NYS, zc = d.zc;
+    const long long base = spectral_base(d, d.NZS, zc - d.NZS * d.nkx), cu = c * d.Ns, cw = both ? 2 * d.Ns : cu;
+    const double *adv = st.ad_v + (long long)zc * d.ncy;
+    double2 f[E], z[E];
+    double ad[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int y = ycoef<E>(e);
+        f[e] = mk(0.0, 0.0);
+        ad[e] = 0.0;
+        if (y > ny) continue;
+        const long long o = base + (long long)y * d.sy;
+        auto pair = [&](const double2 *q) { return mk(q[cu + o].x, q[cw + o].x); };
+        const double2 r = cadd(cadd(cadd(cscale(s.a0, pair(s.u)), cscale(s.a1, pair(s.u_prev))), cscale(s.b0, pair(s.N))),
+                               cscale(s.b1, pair(s.N_prev)));
+        f[e] = cscale(pp.Re, mk(-r.x, -r.y));
+        ad[e] = adv[y];
+    }
+    auto wall = [&](int side) {
+        return mk(s.bc_v[(2 * c + side) * d.ncol + zc].x, s.bc_v[(2 * (both ? 2 : c) + side) * d.ncol + zc].x);
+    };
+    tau_warp<E>(ny, g, pp.a_V[c], pp.b_V[c], true, wall(0), wall(1), st.wn_v[zc], f, z, ad, t.WL, t.WD, t.WR);
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int y = ycoef<E>(e);
+        if (y > ny) continue;
+        const long long o = base + (long long)y * d.sy;   // (v_out may be u_prev: read above)
+        v_out[cu + o].x = z[e].x;
+        if (both) v_out[cw + o].x = z[e].y;
+    }
+}
+// lane_elems on the device
+__device__ __forceinline__ int flux_elems(int ncy) { return ncy <= 32 ? 1 : ncy <= 64 ? 2 : ncy <= 128 ? 4 : 8; }
+__device__ __noinline__ void flux_columns(const Dims &d, const Tables &t, const PhysParams &pp, double g,
+                                          const SolverState &st, const StepArgs &s, double2 *v_out) {
+    const bool both = pp.a_V[0] == pp.a_V[2] && pp.b_V[0] == pp.b_V[2];
+    for (int c = 0; c < (both ? 1 : 3); c += 2) {
+        switch (flux_elems(d.ncy)) {
+        case 1: flux_column<1>(d, t, pp, g, st, s, v_out, c, both); break;
+        case 2: flux_column<2>(d, t, pp, g, st, s, v_out, c, both); break;
+        case 4: flux_column<4>(d, t, pp, g, st, s, v_out, c, both); break;
+        default: flux_column<8>(d, t, pp, g, st, s, v_out, c, both); break;
+        }
+    }
+}
+
+// FLUX: a fixed flow rate (flux_columns; its calls cost a fixed gradient's solve 5 of
+// 138 us in registers, hence an instance of its own)
+template <bool FLUX>
 __global__ void __launch_bounds__(kThreads, 3)
-k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A) {
+k_solve(const __grid_constant__ Dims d, const __grid_constant__ Tables t, const __grid_constant__ PhysParams pp,
+        double g_v, const __grid_constant__ SolverState st, const __grid_constant__ SolveArgs A) {
     chain_begin();
     extern __shared__ double2 tile[];   // [4][ncy][TC]: R_0, R_1, R_2, P; then (WL, WR) and the pivots
     __shared__ double s_wall[3][2][2 * TC];
@@ -374,7 +437,12 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
     cp_async_wait<0>();
     __syncthreads();
 
+    // the (kz, kx) = (0, 0) column (-1: not on this rank); its block
+    const int zc = d.zc;
+    const bool fix_zero = !s.solve_only && zc >= col0 && zc < col0 + TC;
     // ---- chains ------------------------------------------------------------
+    if constexpr (FLUX)
+        if (w == 3 && fix_zero) flux_columns(d, t, pp, g_v, st, s, A.v_out);
     if (w == 0) {
         const double *sum = T + 6 * S;
         double lower, upper;
@@ -481,8 +549,6 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
     // rows g, g + 16, ... all have the parity of g.  Odd-y coefficients take
     // sigma_0 for p, u, w and sigma_1 for v, even-y the reverse; the second
     // response's sign makes c0 + c1 the even p, u, w and odd v coefficient.
-    const int zc = d.zc;   // the (kz, kx) = (0, 0) column (-1: not on this rank)
-    const bool fix_zero = !s.solve_only && zc >= col0 && zc < col0 + TC;
     bool bad = false;
     if (ok) {
         const bool odd = g & 1;
@@ -555,14 +621,19 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
             const double *uu = st.unit;
             double dpdx, dpdz;
             bool pfail = false;
-            if (pp.grad_pre == 1) {
+            if constexpr (!FLUX) {
                 dpdx = pp.gx;
                 dpdz = pp.gz;
             } else {
                 double qx = 0.0, qz = 0.0;
-                for (int y = 2 * lane; y <= ny; y += 64) {
-                    qx += tile[y * TC + lz].x / (double)(y * y - 1);
-                    qz += tile[2 * S + y * TC + lz].x / (double)(y * y - 1);
+                // summed as flux_column holds the column (the order matters there)
+                const double2 *f = A.v_out + spectral_base(d, d.NZS, zc - d.NZS * nkx);
+                const int elems = flux_elems(ncy);
+                for (int e = 0; e < elems && !(lane & 1); ++e) {
+                    const int y = 2 * (elems * (lane >> 1) + e);
+                    if (y > ny) break;
+                    qx += f[(long long)y * d.sy].x / (double)(y * y - 1);
+                    qz += f[2 * d.Ns + (long long)y * d.sy].x / (double)(y * y - 1);
                 }
                 qx = -sum_warp(qx);
                 qz = -sum_warp(qz);
@@ -578,13 +649,17 @@ k_solve(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, SolveArgs A
             }
             for (int y = lane; y <= ny; y += 32) {
                 const double2 pz = tile[3 * S + y * TC + lz];
+                const long long off = spectral_base(d, d.NZS, zc - d.NZS * nkx) + (long long)y * d.sy;
                 double2 u0 = tile[y * TC + lz], u2 = tile[2 * S + y * TC + lz];
+                if (FLUX) {
+                    u0.x = A.v_out[off].x;
+                    u2.x = A.v_out[2 * d.Ns + off].x;
+                }
                 const double2 u1 = y == 0 ? v1w : mk(0.0, 0.0);
                 u0.x += dpdx * uu[y];
                 u2.x += dpdz * uu[ncy + y];
                 bad |= !(isfinite(pz.x) && isfinite(pz.y) && isfinite(u0.x) && isfinite(u0.y) && isfinite(u1.x) &&
                          isfinite(u1.y) && isfinite(u2.x) && isfinite(u2.y));
-                const long long off = spectral_base(d, d.NZS, zc - d.NZS * nkx) + (long long)y * d.sy;
                 A.p_out[off] = pz;
                 A.v_out[off] = u0;
                 A.v_out[d.Ns + off] = u1;
@@ -704,7 +779,8 @@ cudaError_t configure_solver_kernels(const Dims &d) {
     if (e != cudaSuccess) return e;
     e = configure_scan_solve(d);   // (refuses more than 256 Chebyshev coefficients)
     if (e != cudaSuccess) return e;
-    return raise_smem(k_solve, solve_smem(d));
+    e = raise_smem(k_solve<false>, solve_smem(d));
+    return e == cudaSuccess ? raise_smem(k_solve<true>, solve_smem(d)) : e;
 }
 
 void launch_step_solve(const Dims &d, const Tables &t, const PhysParams &pp, double g_v,
@@ -717,7 +793,8 @@ void launch_step_solve(const Dims &d, const Tables &t, const PhysParams &pp, dou
     A.v_out = a.u_out;
     A.step = a;
     const int blocks = (d.ncol + TC - 1) / TC;
-    launch_chained(k_solve, blocks, kThreads, solve_smem(d), s, d, t, pp, g_v, st, A);
+    auto *kernel = pp.grad_pre == 1 || a.solve_only ? k_solve<false> : k_solve<true>;
+    launch_chained(kernel, blocks, kThreads, solve_smem(d), s, d, t, pp, g_v, st, A);
 }
 
 }  // namespace cdns

@@ -1,13 +1,15 @@
 """Results whose rounding order is kept.
 
-In the mixed form every value of the FP64 part is rounded to FP32 once a step, so
-that in a few steps another order of the FP64 operations leaves unrelated FP32 noise:
-1e-6 in dp/dx of a constant flow rate, which is (Q - q) / q_unit with Q - q some 4e-6
-of Q, up to 7e-7 in the pressure.  The golden values
-(golden/golden_rounding_order.npz, written by this file run as a program) are those
-of the library at commit 32f7165; the same order of operations gives the same bits.
-By the chains of solver.cu dp/dx differs by 4e-7 to 3e-6 here and the pressure by 1e-11
-to 2e-7; the bounds leave room for another last bit in a table, not for that."""
+dp/dx of a constant flow rate is (Q - q) / q_unit with Q - q some 4e-6 of Q, so that
+it shows each last bit of the flux q as 5e-11.  In the mixed form every value of the
+FP64 part is rounded to FP32 once a step, so that in a few steps another order of the
+FP64 operations leaves unrelated FP32 noise: 1e-6 in dp/dx, up to 7e-7 in the pressure.
+The golden values (golden/golden_rounding_order.npz, written by this file run as a
+program) are those of the library at commit 32f7165; in the mixed form the same order
+of operations gives the same bits.  By the chains of solver.cu the mixed dp/dx differs
+by 4e-7 to 3e-6 here and the pressure by 1e-11 to 2e-7, and the FP64 dp/dx by 5e-11
+to 2e-10 where its last bits differ at all; the bounds leave room for another last bit
+in a table or in the nonlinear term, not for that."""
 import os
 import sys
 
@@ -30,6 +32,8 @@ MIXED = {
     "gradient_matrix": ((40, 56, 48, 64, 86, 72), "gradient", "rows4", "matrix"),
     "gradient_fft": ((48, 32, 32, 72, 48, 48), "gradient", "rows4", "fft"),
 }
+FP64 = {"fp64_32": (32, 48, 32, 48, 72, 48), "fp64_62": (62, 58, 40, 96, 88, 60), "fp64_102": (102, 28, 52, 162, 46, 81),
+        "fp64_28": (28, 106, 24, 45, 160, 36), "fp64_130": (20, 150, 16, 32, 226, 24)}
 
 
 def field(mesh):
@@ -87,8 +91,18 @@ def test_mixed(name, monkeypatch):
     assert off(p, want[name + "_p"]) <= 1e-12
 
 
+@pytest.mark.parametrize("name", list(FP64))
+def test_fp64_flow_rate(name):
+    """Against 4e-12: 0.08 of one last bit of q."""
+    dpdx, _ = advance(FP64[name], "rate", cdns.PRECISION_FP64, 6)
+    assert off(dpdx, np.load(GOLDEN)[name + "_dpdx"]) <= 4e-12
+
+
 if __name__ == "__main__":
     out = {}
     for n in MIXED:
         out[n + "_dpdx"], out[n + "_p"] = run_mixed(n, os.environ.__setitem__)
+    del os.environ["CDNS_X_STAGE"], os.environ["CDNS_Y_TRANSFORM"]
+    for n in FP64:
+        out[n + "_dpdx"], _ = advance(FP64[n], "rate", cdns.PRECISION_FP64, 6)
     np.savez(sys.argv[1], **out)

@@ -39,6 +39,7 @@ def compare(m, p, nsteps=4, poke=None):
     for k in range(3):
         assert np.linalg.norm(got[..., k] - sim.u[k]) <= 1e-10 * norm
     assert np.linalg.norm(pres - sim.pressure) <= 1e-9 * np.linalg.norm(sim.pressure)
+    return sim, ctx
 
 
 @pytest.mark.parametrize("NYS", [8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 31, 32, 33, 47])
@@ -61,6 +62,19 @@ def test_wall_conditions(NYS, a_V, b_V):
 @pytest.mark.parametrize("NYS", [12, 17])
 def test_constant_flow_rate(NYS):
     compare(*channel(NYS, INDEX_GRAD_PRE=0, DT=1e-3, Re=500.0, V_Microblow0=1e-3))
+
+
+@pytest.mark.parametrize("a_V,b_V", [((1.0, 1.0, 1.0), (0.0, 0.0, 0.0)), ((1.0, 1.0, 0.7), (0.2, 0.0, 0.1))])
+@pytest.mark.parametrize("NYS", [4, 5, 31, 32, 63, 64, 127, 128, 255])
+def test_flux_column(NYS, a_V, b_V):
+    """The zero-mode column whose flux gives dp/dx, at the ends of its rows per lane (1,
+    2, 4 and 8), u and w together and apart.  dp/dx = (Q - q) / q_unit, q_unit some dt Q:
+    a last bit of q is 2.2e-16 / dt = 2.2e-13; 1e-11 for 45 of them after four steps of
+    another order.  With 5 or 6 coefficients the column itself loses four digits (every
+    order of the solve, warp scans and chains, is 1e-10 to 1e-9 off the oracle's): 1e-8."""
+    m, p = channel(NYS, NXS=3, NZS=2, INDEX_GRAD_PRE=0, DT=1e-3, Re=500.0, a_V=a_V, b_V=b_V, V_Microblow0=1e-3)
+    sim, ctx = compare(m, p)
+    assert abs(ctx.dpdx()[0] - sim.dpdx) <= (1e-8 if NYS < 8 else 1e-11)
 
 
 def test_velocity_changes_between_steps():

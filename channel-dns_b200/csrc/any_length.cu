@@ -19,6 +19,7 @@
 #include <algorithm>
 
 #include "cdns_kernels.cuh"
+#include "fast_div.cuh"
 #include "reg_fft.cuh"
 #include "transform_ops.cuh"
 
@@ -62,14 +63,6 @@ template <int MAXR, class Fn> __device__ __forceinline__ void with_radix(int r, 
     }
 }
 constexpr int kRadices[] = {3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 15, 16, 18, 20, 21, 24, 25};
-
-// x / N for 0 <= x, x N < 2^32: umulhi by ceil(2^32 / N)
-struct FastDiv {
-    unsigned m;
-    int n;
-    __device__ __forceinline__ explicit FastDiv(int d) : m(0xffffffffu / (unsigned)d + 1u), n(d) {}
-    __device__ __forceinline__ int operator()(int x) const { return (int)__umulhi((unsigned)x, m); }
-};
 
 // fft2_lines (transforms.cu) with run-time factors: TL lines, one exchange
 // through S[k1][n2][l] (row stride fft2_kstride), at least max(N1, N2) TL threads.

@@ -51,6 +51,13 @@ def test_z_lengths(n):
     check_nonlinear(*mesh(9, 5, n // 3, 21, 8, n))
 
 
+@pytest.mark.parametrize("n", [9, 12, 15, 24, 30, 75, 90, 162, 384])
+def test_no_streamwise_modes(n):
+    """NXS = 0: one line of x (nkx = 1), more output lines per block than points at 9 and 12."""
+    check_nonlinear(*mesh(0, 6, 3, n, 8, 9))
+    check_nonlinear(*mesh(0, 5, 0, n, 12, 15))
+
+
 @pytest.mark.parametrize("nx2,nz2", [(30, 20), (36, 90), (200, 18)])
 def test_full_spectrum(nx2, nz2):
     """Nyquist modes kept (NX2 = 2 NXS, NZ2 = 2 NZS)."""

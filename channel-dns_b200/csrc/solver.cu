@@ -39,14 +39,17 @@ constexpr int TC = kColsPerBlock;     // columns per block
 constexpr int kThreads = 128;         // warp 0: pressure; warps 0-2: velocity; all: staging
 constexpr int kRowGroups = kThreads / TC;
 
+// Loads with a prefetch of the 256-byte neighbourhood.  They read what the kernel before
+// wrote: volatile and with a memory clobber, so that none moves above chain_begin's wait
+// or across a barrier.
 __device__ __forceinline__ double2 ld256(const double2 *p) {
     double2 v;
-    asm("ld.global.L2::256B.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    asm volatile("ld.global.L2::256B.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
     return v;
 }
 __device__ __forceinline__ double ld256(const double *p) {
     double v;
-    asm("ld.global.L2::256B.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    asm volatile("ld.global.L2::256B.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
     return v;
 }
 struct SolveArgs {

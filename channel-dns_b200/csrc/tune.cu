@@ -39,14 +39,20 @@ std::mutex g_mu;
 std::map<std::string, Choice> g_wisdom;
 std::once_flag g_env_import;
 
+// FP64 choices carry the version of the kernels they were timed with: an entry of other
+// kernels (without a version, or another) is kept in the cache and its file, and timed
+// again.  Mixed ones carry none: their x form is part of what a run returns (its FP32
+// rounding), so that a file keeps fixing it.
+constexpr const char *kKernels = "/2";
+
 std::string mesh_key(const cdns_ctx *c) {
     cudaDeviceProp prop{};
     cudaGetDeviceProperties(&prop, c->device);
     const Dims &d = c->d;
     // the device name holds at most 256 characters; seven ints and separators follow
     char buf[256 + 96];
-    std::snprintf(buf, sizeof buf, "%.256s/%d|%d,%d,%d|%d,%d,%d%s", prop.name, prop.multiProcessorCount, d.NX2,
-                  d.NY2, d.NZ2, d.NXS, d.NYS, d.NZS, c->mixed ? "|fp32" : "");
+    std::snprintf(buf, sizeof buf, "%.256s/%d%s|%d,%d,%d|%d,%d,%d%s", prop.name, prop.multiProcessorCount,
+                  c->mixed ? "" : kKernels, d.NX2, d.NY2, d.NZ2, d.NXS, d.NYS, d.NZS, c->mixed ? "|fp32" : "");
     return buf;
 }
 

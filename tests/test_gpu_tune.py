@@ -1,6 +1,8 @@
 """Launch-shape tuning: the choices are valid and cached per mesh, and both
 forms of the Chebyshev transforms (FP64 MMA products and the FFT / DCT-I form)
 meet the reference's golden vectors, whichever the tuner picks."""
+import json
+
 import numpy as np
 import pytest
 
@@ -31,6 +33,30 @@ def test_tuning_is_valid_and_cached(tmp_path):
     a.set_velocity(np.zeros((m.nkz, m.ncy, m.nkx, 3), dtype=np.complex128))
     a.run(1, 3)
     a.synchronize()
+
+
+def test_wisdom_of_other_kernels(tmp_path):
+    """An FP64 entry without the kernels' version was timed with others: it is kept, but
+    the mesh is timed again.  A mixed entry fixes the x form, which its results show."""
+    m, p = channel_case(32)
+    cdns.wisdom_forget()
+    ctx_for(m, p)
+    path = tmp_path / "wisdom.json"
+    cdns.wisdom_export(str(path))
+    key = json.loads(path.read_text())["entries"][0]["key"]
+    name, shape = key.split("|", 1)
+    old = name.rsplit("/", 1)[0] + "|" + shape
+    cdns.wisdom_forget()
+    path.write_text('{"cdns_wisdom": 1, "entries": [{"key": "%s", "ztl": 8, "yform": 0, "xrw": 1}, '
+                    '{"key": "%s|fp32", "ztl": 0, "yform": 0, "xrw": 1}]}\n' % (old, old))
+    cdns.wisdom_import(str(path))
+    ctx_for(m, p)
+    mesh = cdns.Mesh(m.NX, m.NY, m.NZ, m.NXS, m.NYS, m.NZS, m.NX2, m.NY2, m.NZ2, m.XL, m.ZL)
+    mixed = cdns.Context(mesh, cdns.Params(Re=p.Re, DT=p.DT), precision=cdns.PRECISION_MIXED)
+    assert mixed.tuning() == {"z_lines": 0, "y_synthesis": "matrix", "y_analysis": "matrix", "x_rows": 1}
+    cdns.wisdom_export(str(path))
+    assert {e["key"] for e in json.loads(path.read_text())["entries"]} == {key, old, old + "|fp32"}
+    cdns.wisdom_forget()
 
 
 @pytest.mark.parametrize("form", ["matrix", "fft"])

@@ -17,7 +17,7 @@ import numpy as np
 import pytest
 
 import cdns
-from oracle_cases import band_spectrum, channel_case, divergence_free_field
+from oracle_cases import band_spectrum, channel_case, divergence_free_field, orc
 from test_gpu_parity import ctx_for
 
 pytestmark = pytest.mark.gpu
@@ -79,6 +79,25 @@ def test_nonlinear_adjoint_dot_product(n, form, monkeypatch):
     lhs = rdot(lN, Np - Nm) + rdot(lB, Bp - Bm)
     lu = ctx.nonlinear_adjoint(u, lN, lB)
     rhs_ = 2.0 * rdot(lu, d)
+    scale = np.abs(np.conj(lN) * (Np - Nm)).sum() + np.abs(np.conj(lB) * (Bp - Bm)).sum()
+    assert abs(lhs - rhs_) <= 1e-11 * scale, (lhs, rhs_, scale)
+
+
+@pytest.mark.parametrize("ny2,nys", [(12, 7), (30, 20), (90, 59), (162, 107), (252, 167), (384, 255)])
+def test_nonlinear_adjoint_run_time_factors(ny2, nys, monkeypatch):
+    """The same identity with Chebyshev lengths of the run-time-factor kernel (largest
+    factor up to 16, 20 and 25) and small x and z lengths of its kind."""
+    monkeypatch.setenv("CDNS_Y_TRANSFORM", "fft")
+    m = orc.Mesh(12, ny2, 10, 6, nys, 5, 18, ny2, 15, 4.0 * np.pi, 2.0 * np.pi)
+    ctx = ctx_for(m, orc.Parm(Re=180.0, DT=5e-5))
+    assert ctx.tuning()["y_synthesis"] == "fft"
+    u, d = (np.stack([band_spectrum(m, seed=s + c, amp=0.05) for c in range(3)], axis=-1) for s in (5, 20))
+    rng = np.random.default_rng(ny2)
+    lN, lB = crandom(rng, u.shape), crandom(rng, (m.nkz, 2, m.nkx))
+    Np, Bp = ctx.nonlinear(u + d)
+    Nm, Bm = ctx.nonlinear(u - d)
+    lhs = rdot(lN, Np - Nm) + rdot(lB, Bp - Bm)
+    rhs_ = 2.0 * rdot(ctx.nonlinear_adjoint(u, lN, lB), d)
     scale = np.abs(np.conj(lN) * (Np - Nm)).sum() + np.abs(np.conj(lB) * (Bp - Bm)).sum()
     assert abs(lhs - rhs_) <= 1e-11 * scale, (lhs, rhs_, scale)
 

@@ -2,6 +2,8 @@
 numbers advanced together (steady steps as one graph of parallel branches)
 give, member by member, exactly the fields of the same channel run alone;
 member errors are reported with their index."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -67,6 +69,34 @@ def test_batch_continues_after_more_steps():
     b.synchronize()
     for x, y in zip(a.members, b.members):
         assert np.array_equal(x.get_velocity(), y.get_velocity())
+
+
+@pytest.mark.parametrize("precision", [cdns.PRECISION_FP64, cdns.PRECISION_MIXED])
+def test_contexts_on_threads(precision):
+    """Channels created and stepped by a thread each, side by side on their own streams
+    (setup, plain launches, capture and replay of chained launches): the fields of the
+    same channels one after the other, bit for bit."""
+    mp = [mesh_params(n, re) for n, re in MEMBERS]
+    u0 = fields(MEMBERS)
+
+    def advance(k, out):
+        ctx = cdns.Context(mp[k][2], mp[k][3], precision=precision)
+        ctx.set_velocity(u0[k])
+        for it in range(1, 41):
+            ctx.step(it)
+        ctx.synchronize()
+        out[k] = ctx.get_velocity()
+
+    alone, beside = {}, {}
+    for k in range(len(MEMBERS)):   # also fixes the tuned shapes of each mesh
+        advance(k, alone)
+    threads = [threading.Thread(target=advance, args=(k, beside)) for k in range(len(MEMBERS))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(len(MEMBERS)):
+        assert np.array_equal(alone[k], beside[k])
 
 
 def test_batch_reports_member_error():

@@ -155,6 +155,26 @@ def test_mixed_rejects_meshes_without_register_form(key):
         mixed_ctx_for(m, p)
 
 
+@pytest.mark.parametrize("shape", [(48, 84, 112, 72, 126, 192), (120, 64, 60, 192, 98, 96), (32, 32, 32, 48, 48, 48)])
+@pytest.mark.parametrize("flow", ["rate", "gradient"])
+def test_mixed_pressure_and_gradient(shape, flow):
+    """What the mixed form gives beside the velocity, eight steps: dp/dx of a constant flow
+    rate divides FP32 noise of the mean flux by the flux of a unit gradient over one step
+    and is good to 1e-5 (1e-6 to 6e-6 seen over 24 to 128 points a side), the pressure to
+    3e-6 (1e-7 to 8e-7 seen); the velocity to 1e-7 (1e-9 to 3e-8 seen)."""
+    nx, ny, nz, nx2, ny2, nz2 = shape
+    box = (10.0, 10.0) if flow == "rate" else (4.0 * np.pi, 2.0 * np.pi)
+    m = orc.Mesh(nx, ny, nz, nx // 2, ny - 2, nz // 2, nx2, ny2, nz2, *box)
+    p = orc.Parm(Re=2800.0, DT=3e-3, INDEX_GRAD_PRE=0, V_Microblow0=1e-3) if flow == "rate" else orc.Parm(Re=180.0, DT=5e-5)
+    u0 = divergence_free_field(m, p, seed=3, amp=0.1, spectrum="k53", mean="laminar" if flow == "rate" else "loglaw")
+    ctxs = [ctx_for(m, p), mixed_ctx_for(m, p)]
+    u64, u32 = (run(c, u0, 8) for c in ctxs)
+    (g64, p64), (g32, p32) = ((np.array(c.dpdx()), c.get_pressure()) for c in ctxs)
+    assert rel_l2(u32, u64) <= 1e-7
+    assert rel_l2(p32, p64) <= 3e-6
+    assert rel_l2(g32, g64) <= 1e-5
+
+
 @pytest.mark.parametrize("form", ["matrix", "fft"])
 def test_mixed_chebyshev_forms(form, monkeypatch):
     """Both forms of the Chebyshev transforms on the FP32 stage buffers (the

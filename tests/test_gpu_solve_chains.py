@@ -1,5 +1,5 @@
-"""The column solve's chains (csrc/solver.cu) at the ends of their row groups:
-every NYS from the smallest up, column counts that do not fill a block, both
+"""The column solve's chains (csrc/solver.cu) at the ends of their row groups: the
+smallest NYS and some up to the largest, column counts that do not fill a block, both
 forcings, wall conditions that differ between u and w, and the curl that the
 solve leaves for the next step (changes of the velocity between steps).  Time
 steps against the oracle's loop at the step tolerance (relative L2 <= 1e-10)."""
@@ -45,6 +45,13 @@ def compare(m, p, nsteps=4, poke=None):
 @pytest.mark.parametrize("NYS", [8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 31, 32, 33, 47])
 def test_rows(NYS):
     compare(*channel(NYS))
+
+
+@pytest.mark.parametrize("NYS", [4, 5, 6, 7, 254, 255])
+def test_rows_smallest_and_largest(NYS):
+    """4 to 7: no full group of rows, the two top rows next to y = 2, row groups without a
+    row.  254 and 255: the largest tile and every held pivot."""
+    compare(*channel(NYS, NXS=4, NZS=3))
 
 
 @pytest.mark.parametrize("NXS,NZS", [(0, 3), (1, 1), (3, 0), (4, 2), (8, 9)])

@@ -59,23 +59,24 @@ def workload_mesh():
 
 
 def stage_bytes(mesh):
-    """Algorithmic HBM bytes per launch of each stage (16 B per complex value;
-    every stage reads and writes its operands once)."""
+    """Algorithmic HBM bytes per launch of each stage of a steady FP64 step (16 B per
+    complex value; every stage reads and writes its operands once)."""
     nkx, nkz, ncy = mesh.NXS + 1, 2 * mesh.NZS + 1, mesh.NYS + 1
     ny2 = mesh.NY2 + 1
     Ns = nkz * ncy * nkx
     Ny = nkz * ny2 * nkx
     Nz = mesh.NZ2 * ny2 * nkx
     return {
-        "curl": 16 * (3 * Ns + 3 * Ns),
+        "curl": 0,   # no launch: the solve leaves the curl of the new velocity
         "y_synthesis": 16 * (6 * Ns + 6 * Ny),
         "z_backward": 16 * 6 * (Ny + Nz),
         "x_cross": 16 * 9 * Nz,
         "z_forward": 16 * 3 * (Nz + Ny),
         "y_analysis": 16 * (3 * Ny + 3 * Ns),
-        # R from u, u_prev, N, N_prev (12), influence + B-problem fields (12),
-        # tau pivots ad_p, ad_v (1 complex-equivalent), writes u, p (4)
-        "solve": 16 * 29 * Ns,
+        # reads u, u_prev, N, N_prev (12) and, over the columns kz <= 0, three real
+        # influence and three B-problem fields and the pivots ad_p, ad_v; writes u, p
+        # and the vorticity (7)
+        "solve": 16 * 19 * Ns + 8 * 8 * (mesh.NZS + 1) * ncy * nkx,
     }
 
 
@@ -88,7 +89,7 @@ STAGE_SOURCES = {
     "x_cross": ["transforms.cu", "reg_fft.cuh", "fft_lines.cuh", "transform_ops.cuh"],
     "z_forward": ["transforms.cu", "reg_fft.cuh", "fft_lines.cuh", "transform_ops.cuh"],
     "y_analysis": ["chebyshev.cu", "transforms.cu", "reg_fft.cuh", "transform_ops.cuh"],
-    "solve": ["solver.cu", "warp_columns.cuh"],
+    "solve": ["solver.cu", "tau_warp.cuh", "warp_columns.cuh"],
 }
 TRAFFIC_PROFILE = os.path.join(ROOT, "profiles", "dram_traffic_retau180.md")
 
@@ -794,7 +795,7 @@ def main():
                     "protocol": "upload + steps 1..K (setup included) one call each with dpdx readback + download"},
             "clocks": clk,
             "setup_steps": {"ms": setup_ms, "steps": 2},
-            "gpu_launches": len(per_launch) * K,   # one kernel per stage per step
+            "gpu_launches": sum(1 for b in sb.values() if b) * K,   # one kernel per stage per step
         }
         print(json.dumps(_rounded(line)), flush=True)
         if args.detail:

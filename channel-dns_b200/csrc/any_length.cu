@@ -8,10 +8,11 @@
 // 384), these one exchange per transform with the radix code straight-line.
 // The lengths that the switch does not cover (a prime factor above 7, or no
 // split into two factors of at most 25) keep the Stockham form.  A step of 60 x 51 x
-// 54 takes 106 us instead of 162, one of 256 x 193 x 192 2.9 ms instead of 7.1 (x
+// 66 takes 67 us instead of 150, one of 256 x 193 x 192 2.9 ms instead of 7.1 (x
 // stage of 384 points 1.12 instead of 2.94, z of 288 0.53 instead of 1.24, y of 288
 // 0.75 instead of 1.56 as matrix products).  Bound by latency at the warps that the
-// registers leave, and by the shared-memory pipe.
+// registers leave, and by the shared-memory pipe.  FP32 stages take none of these
+// (their x and z lengths all have compiled splits; why not y: solver_scan.cu).
 //
 // Three instances of each kernel, by the largest factor (16, 20 or 25): a DFT of
 // 20 needs some 20 registers more than one of 16, one of 24 another 30, and the

@@ -614,7 +614,8 @@ void launch_yanalysis_scaled(const Dims &d, const double *cana, const double2 *F
 
 void launch_mean_products(const Dims &d, const Tables &t, const double *mean, double2 *S, cudaStream_t s) {
     const int warps = 3 * d.ncy, per_block = 8;
-    launch_chained(k_mean_products, (warps + per_block - 1) / per_block, 32 * per_block, sizeof(double) * 3 * d.ny2, s, d, t.cana, ana_groups(d) * kAnaRows, mean, S);
+    launch_chained(k_mean_products, (warps + per_block - 1) / per_block, 32 * per_block, sizeof(double) * 3 * d.ny2, s, d,
+                   t.cana, ana_groups(d) * kAnaRows, mean, S);
 }
 
 }  // namespace cdns

@@ -386,8 +386,8 @@ int create_context(const cdns_mesh_desc *m, const cdns_params *p, int precision,
     if ((r = c->alloc(c->U[0], 3 * Ns)) || (r = c->alloc(c->U[1], 3 * Ns)) ||
         (r = c->alloc(c->Nb[0], 3 * Ns)) || (r = c->alloc(c->Nb[1], 3 * Ns)) ||
         (r = c->alloc(c->Bb[0], 2 * nc)) || (r = c->alloc(c->Bb[1], 2 * nc)) ||
-        (r = c->alloc(c->p, Ns)) || (r = c->alloc(c->bwb[0], 2 * nc)) || (r = c->alloc(c->bwb[1], 2 * nc)) || (r = c->alloc(c->bc_v, 6 * nc)) ||
-        (r = c->alloc(c->bc_p, 2 * nc)) || (r = c->alloc(c->F, fbuf)) || (r = c->alloc(c->G, gbuf)) ||
+        (r = c->alloc(c->p, Ns)) || (r = c->alloc(c->bwb[0], 2 * nc)) || (r = c->alloc(c->bwb[1], 2 * nc)) ||
+        (r = c->alloc(c->bc_v, 6 * nc)) || (r = c->alloc(c->bc_p, 2 * nc)) || (r = c->alloc(c->F, fbuf)) || (r = c->alloc(c->G, gbuf)) ||
         (r = c->alloc(c->H, hbuf)) || (r = c->alloc(c->aux, 3 * Ns)) || (r = c->alloc(c->aux2, 3 * Ns)) ||
         (r = c->alloc(c->zero3, 3 * Ns)) || (r = c->alloc(c->om, 3 * Ns)) ||
         (r = c->alloc(c->mean, 6 * (size_t)d.ny2)) ||

@@ -5,9 +5,9 @@
 // derivative recurrence (src/solver/vector_ops.cpp:17-25) couples only
 // coefficients of one parity of y, and its multipliers are real: a column is
 // four independent scalar chains per field, (parity, re/im).  One thread runs
-// one chain sequentially over columns staged in shared memory: a block holds TC consecutive columns, a warp the 4 TC chains of
-// one field, so that a row of the tile is read by 16 lanes as 128 consecutive
-// bytes.  The whole solve is two sweeps down and up the chain for the pressure
+// one chain sequentially over columns staged in shared memory: a block holds TC
+// consecutive columns, a warp the 4 TC chains of one field, so that a row of the
+// tile is read by 16 lanes as 128 consecutive bytes.  The whole solve is two sweeps down and up the chain for the pressure
 // (one warp) and two for the velocity (three warps, one per component); the
 // right-hand sides (divergence of R, Re (grad P - R)) are formed inside the
 // downward sweep and the wall sums inside the upward one.
@@ -22,6 +22,9 @@
 //   - u and w are i kx phi and i kz phi of one phi where u and w have the same
 //     wall condition, so one of the two gives the other;
 //   - column -kz has the same pressure, u, v and pivots and w negated.
+// Two things keep the warp scans that this form replaced, because the order of the
+// operations shows in what they give: the mixed form (solver_scan.cu) and the column
+// whose flux gives dp/dx (flux_column).
 // The curl of the new velocity (vector_ops.cpp:112-151) and its wall sums are
 // formed from the columns while they are in shared memory.
 // What bounds it: the chains' latency at 12 warps per SM against the streams
@@ -267,9 +270,9 @@ template <int C> struct VelocityRhs {
 // operations is part of the result: by the chains, dp/dx of a 32 x 49 x 32 channel is
 // 5e-11 to 1e-10 off after six steps.  No pressure enters (kx = kz = 0), nor do the
 // corrections.  Warp 3 of one block does it beside the pressure chains: a step of 32 x
-// 33 x 32 takes 36.9 us with it and without (41.0 with u and w one after the other
-// beside the velocity chains).  (u, w) are one double2 column where their wall conditions
-// are the same (c = 0, both), else one after the other.
+// 33 x 32 takes 17.1 us with it, 17.0 without (4 us more with u and w one after the
+// other beside the velocity chains).  (u, w) are one double2 column where their wall
+// conditions are the same (c = 0, both), else one after the other.
 template <int E>
 __device__ __noinline__ void flux_column(const Dims &d, const Tables &t, const PhysParams &pp, double g,
                                          const SolverState &st, const StepArgs &s, double2 *v_out, int c, bool both) {
@@ -286,7 +289,8 @@ __device__ __noinline__ void flux_column(const Dims &d, const Tables &t, const P
         if (y > ny) continue;
         const long long o = base + (long long)y * d.sy;
         auto pair = [&](const double2 *q) { return mk(q[cu + o].x, q[cw + o].x); };
-        const double2 r = cadd(cadd(cadd(cscale(s.a0, pair(s.u)), cscale(s.a1, pair(s.u_prev))), cscale(s.b0, pair(s.N))),
+        const double2 r = cadd(cadd(cadd(cscale(s.a0, pair(s.u)), cscale(s.a1, pair(s.u_prev))),
+                                    cscale(s.b0, pair(s.N))),
                                cscale(s.b1, pair(s.N_prev)));
         f[e] = cscale(pp.Re, mk(-r.x, -r.y));
         ad[e] = adv[y];
@@ -726,7 +730,8 @@ k_solve(const __grid_constant__ Dims d, const __grid_constant__ Tables t, const 
             const int sl = y * TC + l;
             const long long o = out0 + (long long)y * d.sy;
             const double2 v = tile[S + sl];
-            const double2 du = y < ny ? tile[sl + TC] : mk(0.0, 0.0), dw = y < ny ? tile[2 * S + sl + TC] : mk(0.0, 0.0);
+            const double2 du = y < ny ? tile[sl + TC] : mk(0.0, 0.0);
+            const double2 dw = y < ny ? tile[2 * S + sl + TC] : mk(0.0, 0.0);
             s.om[o] = csub(dw, fderiv(azl, v));
             s.om[2 * d.Ns + o] = csub(fderiv(axl, v), du);
         }

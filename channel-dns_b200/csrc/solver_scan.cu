@@ -315,8 +315,8 @@ cudaError_t configure_scan_solve(const Dims &d) {
 void launch_scan_solve(const Dims &d, const Tables &t, const PhysParams &pp, double g_v, const SolverState &st,
                        const StepArgs &a, cudaStream_t s) {
     with_elems(d, [&](auto n) {
-        launch_chained(k_solve_scan<decltype(n)::value>, (d.ncol + TC - 1) / TC, kThreads, scan_smem(d), s, d, t, pp, g_v,
-                       st, a);
+        launch_chained(k_solve_scan<decltype(n)::value>, (d.ncol + TC - 1) / TC, kThreads, scan_smem(d), s, d, t, pp,
+                       g_v, st, a);
     });
 }
 

@@ -379,7 +379,8 @@ cudaError_t configure_setup_kernels(const Dims &d) {
 void setup_solver(const Dims &d, const Tables &t, const PhysParams &pp, double g_v, SolverState &st,
                   double2 *, cudaStream_t s) {
     const int nb = (d.ncol + 127) / 128;
-    k_wn_ad<<<dim3(((d.NZS + 1) * d.nkx * 2 + 127) / 128, 2), 128, 0, s>>>(d, t, pp.G_pre, g_v, st.wn_p, st.ad_p, st.wn_v, st.ad_v);
+    k_wn_ad<<<dim3(((d.NZS + 1) * d.nkx * 2 + 127) / 128, 2), 128, 0, s>>>(d, t, pp.G_pre, g_v, st.wn_p, st.ad_p, st.wn_v,
+                                                                           st.ad_v);
     const int blocks = ((d.NZS + 1) * d.nkx + TC - 1) / TC;   // columns kz <= 0
     const size_t sm = setup_smem(d);
     // influence responses: pressure Dirichlet data (1,0) and (0,1), in one launch

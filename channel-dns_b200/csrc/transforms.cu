@@ -1758,7 +1758,8 @@ bool z_backward_r(const Dims &d, const double2 *roots, const C *F, C *G, int nf,
     dim3 grid((d.nkx + tl - 1) / tl, d.ny2, nf);
     return with_xsplit(d.NZ2, [&](auto a, auto b) {
         constexpr int N1 = decltype(a)::value, N2 = decltype(b)::value;
-        launch_chained(k_z_backward_r<N1, N2, C>, grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(C)), s, d, roots, F, G, tl, coarse);
+        launch_chained(k_z_backward_r<N1, N2, C>, grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(C)), s,
+                       d, roots, F, G, tl, coarse);
     });
 }
 template <class C, bool MEAN>
@@ -1780,11 +1781,13 @@ bool x_cross_r(const Dims &d, const double2 *roots, const C *G, C *H, const doub
             if (d.xrw == 3 || d.xrw == 5) {   // 4 or 2 rows, forward phases split over lane pairs
                 const int srw = d.xrw == 3 ? 4 : 2;
                 dim3 sgrid((d.NZ2 + srw - 1) / srw, d.ny2);
-                launch_chained(k_x_cross_r<N1, N2, C, MEAN, true>, sgrid, 16 * 3 * srw, smem_xcross_r(N1, N2, sizeof(C), srw), s, d, roots, G, H, srw, mean);
+                launch_chained(k_x_cross_r<N1, N2, C, MEAN, true>, sgrid, 16 * 3 * srw, smem_xcross_r(N1, N2, sizeof(C), srw), s,
+                               d, roots, G, H, srw, mean);
                 return;
             }
         }
-        launch_chained(k_x_cross_r<N1, N2, C, MEAN>, grid, 16 * 3 * rw, smem_xcross_r(N1, N2, sizeof(C)), s, d, roots, G, H, rw, mean);
+        launch_chained(k_x_cross_r<N1, N2, C, MEAN>, grid, 16 * 3 * rw, smem_xcross_r(N1, N2, sizeof(C)), s,
+                       d, roots, G, H, rw, mean);
     });
 }
 template <class C>
@@ -1794,7 +1797,8 @@ bool z_forward_r(const Dims &d, const double2 *roots, const C *H, C *F, int nf, 
     dim3 grid((d.nkx + tl - 1) / tl, d.ny2, nf);
     return with_xsplit(d.NZ2, [&](auto a, auto b) {
         constexpr int N1 = decltype(a)::value, N2 = decltype(b)::value;
-        launch_chained(k_z_forward_r<N1, N2, C>, grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(C)), s, d, roots, H, F, tl, coarse);
+        launch_chained(k_z_forward_r<N1, N2, C>, grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(C)), s,
+                       d, roots, H, F, tl, coarse);
     });
 }
 
@@ -1804,7 +1808,8 @@ bool launch_z_backward_peers(const Dims &d, const double2 *roots, const PeerCols
     dim3 grid((d.nkx + tl - 1) / tl, d.ny2, 6);
     return with_xsplit(d.NZ2, [&](auto a, auto b) {
         constexpr int N1 = decltype(a)::value, N2 = decltype(b)::value;
-        launch_chained(k_z_backward_peers<N1, N2>, grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(double2)), s, d, roots, pc, G, tl);
+        launch_chained(k_z_backward_peers<N1, N2>, grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(double2)), s,
+                       d, roots, pc, G, tl);
     });
 }
 
@@ -1814,7 +1819,8 @@ bool launch_z_forward_peers(const Dims &d, const double2 *roots, const double2 *
     dim3 grid((d.nkx + tl - 1) / tl, d.ny2, 3);
     return with_xsplit(d.NZ2, [&](auto a, auto b) {
         constexpr int N1 = decltype(a)::value, N2 = decltype(b)::value;
-        launch_chained(k_z_forward_peers<N1, N2>, grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(double2)), s, d, roots, H, pc, tl);
+        launch_chained(k_z_forward_peers<N1, N2>, grid, (N1 > N2 ? N1 : N2) * tl, smem_zfft_r(d, N1, N2, sizeof(double2)), s,
+                       d, roots, H, pc, tl);
     });
 }
 

@@ -52,7 +52,13 @@ typedef enum {
  * FP32 (the y synthesis/analysis accumulate in FP64 and round to or from FP32
  * at the stage boundary); the curl, the tau solves, the influence and sigma
  * corrections, the pressure wall data and the mean-flow update stay FP64.
- * MIXED needs NX2 and NZ2 in {32, 48, 64, 72, 96, 128, 144, 192, 196}. */
+ * MIXED needs NX2 and NZ2 in {32, 48, 64, 72, 96, 128, 144, 192, 196}.
+ * Against FP64, after 3 to 8 steps: the velocity differs by up to 3e-8
+ * (relative L2), the pressure by up to 8e-7, and dp/dx of a constant flow rate
+ * (INDEX_GRAD_PRE = 0) by up to 6e-6, since it divides the FP32 noise of the
+ * mean flux by what a unit gradient adds to it in one step.  A run's bits
+ * depend on the x-stage form (cdns_get_tuning), which is timed: CDNS_X_STAGE, or
+ * a wisdom file, makes dp/dx and the pressure repeat between processes. */
 typedef enum { CDNS_PRECISION_FP64 = 0, CDNS_PRECISION_MIXED = 1 } cdns_precision;
 
 /* Mesh, mirrors MeshParm (src/core/params.hpp:6-11) + XL/ZL
@@ -234,7 +240,9 @@ int cdns_solve(cdns_ctx *ctx, double g, const double *rhs_velocity, const double
  * (x-stage form: 4 or 2 rows per block, 1 the half-warp form, 3 or 5 the
  * lane-pair split form with 4 or 2 rows);
  * cdns_wisdom_export / _import save and load the choices as JSON (host-only
- * calls); cdns_wisdom_forget empties the process cache. */
+ * calls); cdns_wisdom_forget empties the process cache.  FP64 entries carry the
+ * version of the kernels they were timed with: others are kept, and their mesh
+ * is timed again. */
 int cdns_tune(cdns_ctx *ctx);
 int cdns_get_tuning(cdns_ctx *ctx, int *out);
 int cdns_wisdom_export(const char *path);

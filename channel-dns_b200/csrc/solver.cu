@@ -24,7 +24,7 @@
 //   - column -kz has the same pressure, u, v and pivots and w negated.
 // Two things keep the warp scans that this form replaced, because the order of the
 // operations shows in what they give: the mixed form (solver_scan.cu) and the column
-// whose flux gives dp/dx (flux_column).
+// that gives dp/dx and the mean wall shear (flux_column).
 // The curl of the new velocity (vector_ops.cpp:112-151) and its wall sums are
 // formed from the columns while they are in shared memory.
 // What bounds it: the chains' latency at 12 warps per SM against the streams
@@ -264,17 +264,19 @@ template <int C> struct VelocityRhs {
 };
 
 // The real parts of u and w of the (kz, kx) = (0, 0) column before their pressure
-// gradient, by warp scans and from the multistep state: the column whose fluxes give
-// dp/dx and dp/dz where the flow rate is fixed.  dp/dx = (Q - q) / q_unit, with Q - q
-// some 4e-6 of Q, shows each last bit of this column as 5e-11, so that the order of its
-// operations is part of the result: by the chains, dp/dx of a 32 x 49 x 32 channel is
-// 5e-11 to 1e-10 off after six steps.  No pressure enters (kx = kz = 0), nor do the
-// corrections.  Warp 3 of one block does it beside the pressure chains: a step of 32 x
-// 33 x 32 takes 17.1 us with it, 17.0 without (4 us more with u and w one after the
-// other beside the velocity chains).  (u, w) are one double2 column where their wall
-// conditions are the same (c = 0, both), else one after the other.
+// gradient, by warp scans and from the multistep state: the column that gives dp/dx and
+// dp/dz where the flow rate is fixed, and the mean wall shear.  dp/dx = (Q - q) / q_unit,
+// with Q - q some 4e-6 of Q, shows each last bit of it as 5e-11, and the shear weights
+// coefficient k by k^2, so that the order of its operations is part of the result: by
+// the chains, dp/dx of a 32 x 49 x 32 channel is 5e-11 to 1e-10 off after six steps, the
+// mean shear of a 50 x 27 x 40 one 7e-12 after twelve.  No pressure enters (kx = kz = 0),
+// nor do the corrections.  Warp 3 of one block does it beside the pressure chains.  That
+// block is the first to start: with it among the last, its 4 to 7 us more were the
+// kernel's (144 us instead of 138 at 128 x 129 x 128, 547 instead of 528 at 256 x 193 x
+// 192).  (u, w) are one double2 column where their wall conditions are the same (c = 0,
+// both), else one after the other.
 template <int E>
-__device__ __noinline__ void flux_column(const Dims &d, const Tables &t, const PhysParams &pp, double g,
+__device__ __forceinline__ void flux_column(const Dims &d, const Tables &t, const PhysParams &pp, double g,
                                          const SolverState &st, const StepArgs &s, double2 *v_out, int c, bool both) {
     const int ny = d.NYS, zc = d.zc;
     const long long base = spectral_base(d, d.NZS, zc - d.NZS * d.nkx), cu = c * d.Ns, cw = both ? 2 * d.Ns : cu;
@@ -308,24 +310,7 @@ __device__ __noinline__ void flux_column(const Dims &d, const Tables &t, const P
         if (both) v_out[cw + o].x = z[e].y;
     }
 }
-// lane_elems on the device
-__device__ __forceinline__ int flux_elems(int ncy) { return ncy <= 32 ? 1 : ncy <= 64 ? 2 : ncy <= 128 ? 4 : 8; }
-__device__ __noinline__ void flux_columns(const Dims &d, const Tables &t, const PhysParams &pp, double g,
-                                          const SolverState &st, const StepArgs &s, double2 *v_out) {
-    const bool both = pp.a_V[0] == pp.a_V[2] && pp.b_V[0] == pp.b_V[2];
-    for (int c = 0; c < (both ? 1 : 3); c += 2) {
-        switch (flux_elems(d.ncy)) {
-        case 1: flux_column<1>(d, t, pp, g, st, s, v_out, c, both); break;
-        case 2: flux_column<2>(d, t, pp, g, st, s, v_out, c, both); break;
-        case 4: flux_column<4>(d, t, pp, g, st, s, v_out, c, both); break;
-        default: flux_column<8>(d, t, pp, g, st, s, v_out, c, both); break;
-        }
-    }
-}
-
-// FLUX: a fixed flow rate (flux_columns; its calls cost a fixed gradient's solve 5 of
-// 138 us in registers, hence an instance of its own)
-template <bool FLUX>
+template <int E>
 __global__ void __launch_bounds__(kThreads, 3)
 k_solve(const __grid_constant__ Dims d, const __grid_constant__ Tables t, const __grid_constant__ PhysParams pp,
         double g_v, const __grid_constant__ SolverState st, const __grid_constant__ SolveArgs A) {
@@ -338,8 +323,10 @@ k_solve(const __grid_constant__ Dims d, const __grid_constant__ Tables t, const 
     const int AS = pivot_stride(ncy);
     double2 *s_w = tile + 3 * S + max(ncy, kRowGroups) * TC;         // [ncy] (WL, WR)
     double *s_ad = reinterpret_cast<double *>(s_w + ncy);             // [TC][AS]
-    // blocks of kz and -kz next to each other: from both ends inwards
-    const int blk = (blockIdx.x & 1) ? (int)gridDim.x - 1 - (int)(blockIdx.x >> 1) : (int)(blockIdx.x >> 1);
+    // blocks of kz and -kz next to each other: from the middle outwards, so that the block
+    // with flux_column's work starts first
+    const int bi = (int)gridDim.x - 1 - (int)blockIdx.x;
+    const int blk = (bi & 1) ? (int)gridDim.x - 1 - (bi >> 1) : (bi >> 1);
     const int col0 = blk * TC;
     const int tid = threadIdx.x;
     const int w = tid >> 5, lane = tid & 31;
@@ -448,8 +435,11 @@ k_solve(const __grid_constant__ Dims d, const __grid_constant__ Tables t, const 
     const int zc = d.zc;
     const bool fix_zero = !s.solve_only && zc >= col0 && zc < col0 + TC;
     // ---- chains ------------------------------------------------------------
-    if constexpr (FLUX)
-        if (w == 3 && fix_zero) flux_columns(d, t, pp, g_v, st, s, A.v_out);
+    if (w == 3 && fix_zero) {
+        const bool both = pp.a_V[0] == pp.a_V[2] && pp.b_V[0] == pp.b_V[2];
+#pragma unroll 1
+        for (int c = 0; c < (both ? 1 : 3); c += 2) flux_column<E>(d, t, pp, g_v, st, s, A.v_out, c, both);
+    }
     if (w == 0) {
         const double *sum = T + 6 * S;
         double lower, upper;
@@ -628,16 +618,15 @@ k_solve(const __grid_constant__ Dims d, const __grid_constant__ Tables t, const 
             const double *uu = st.unit;
             double dpdx, dpdz;
             bool pfail = false;
-            if constexpr (!FLUX) {
+            if (pp.grad_pre == 1) {
                 dpdx = pp.gx;
                 dpdz = pp.gz;
             } else {
                 double qx = 0.0, qz = 0.0;
                 // summed as flux_column holds the column (the order matters there)
                 const double2 *f = A.v_out + spectral_base(d, d.NZS, zc - d.NZS * nkx);
-                const int elems = flux_elems(ncy);
-                for (int e = 0; e < elems && !(lane & 1); ++e) {
-                    const int y = 2 * (elems * (lane >> 1) + e);
+                for (int e = 0; e < E && !(lane & 1); ++e) {
+                    const int y = 2 * (E * (lane >> 1) + e);
                     if (y > ny) break;
                     qx += f[(long long)y * d.sy].x / (double)(y * y - 1);
                     qz += f[2 * d.Ns + (long long)y * d.sy].x / (double)(y * y - 1);
@@ -658,10 +647,8 @@ k_solve(const __grid_constant__ Dims d, const __grid_constant__ Tables t, const 
                 const double2 pz = tile[3 * S + y * TC + lz];
                 const long long off = spectral_base(d, d.NZS, zc - d.NZS * nkx) + (long long)y * d.sy;
                 double2 u0 = tile[y * TC + lz], u2 = tile[2 * S + y * TC + lz];
-                if (FLUX) {
-                    u0.x = A.v_out[off].x;
-                    u2.x = A.v_out[2 * d.Ns + off].x;
-                }
+                u0.x = A.v_out[off].x;
+                u2.x = A.v_out[2 * d.Ns + off].x;
                 const double2 u1 = y == 0 ? v1w : mk(0.0, 0.0);
                 u0.x += dpdx * uu[y];
                 u2.x += dpdz * uu[ncy + y];
@@ -787,8 +774,8 @@ cudaError_t configure_solver_kernels(const Dims &d) {
     if (e != cudaSuccess) return e;
     e = configure_scan_solve(d);   // (refuses more than 256 Chebyshev coefficients)
     if (e != cudaSuccess) return e;
-    e = raise_smem(k_solve<false>, solve_smem(d));
-    return e == cudaSuccess ? raise_smem(k_solve<true>, solve_smem(d)) : e;
+    with_elems(d, [&](auto n) { e = raise_smem(k_solve<decltype(n)::value>, solve_smem(d)); });
+    return e;
 }
 
 void launch_step_solve(const Dims &d, const Tables &t, const PhysParams &pp, double g_v,
@@ -801,8 +788,9 @@ void launch_step_solve(const Dims &d, const Tables &t, const PhysParams &pp, dou
     A.v_out = a.u_out;
     A.step = a;
     const int blocks = (d.ncol + TC - 1) / TC;
-    auto *kernel = pp.grad_pre == 1 || a.solve_only ? k_solve<false> : k_solve<true>;
-    launch_chained(kernel, blocks, kThreads, solve_smem(d), s, d, t, pp, g_v, st, A);
+    with_elems(d, [&](auto n) {
+        launch_chained(k_solve<decltype(n)::value>, blocks, kThreads, solve_smem(d), s, d, t, pp, g_v, st, A);
+    });
 }
 
 }  // namespace cdns

@@ -293,17 +293,6 @@ k_solve_scan(Dims d, Tables t, PhysParams pp, double g_v, SolverState st, StepAr
 }
 
 size_t scan_smem(const Dims &d) { return sizeof(double2) * 4 * (size_t)d.ncy * TC; }
-
-// fn(E) for the elements per lane of this column length
-template <class Fn> bool with_elems(const Dims &d, Fn &&fn) {
-    switch (lane_elems(d)) {
-    case 1: fn(std::integral_constant<int, 1>{}); return true;
-    case 2: fn(std::integral_constant<int, 2>{}); return true;
-    case 4: fn(std::integral_constant<int, 4>{}); return true;
-    case 8: fn(std::integral_constant<int, 8>{}); return true;
-    default: return false;   // more than 256 Chebyshev coefficients
-    }
-}
 }  // namespace
 
 cudaError_t configure_scan_solve(const Dims &d) {

@@ -11,6 +11,8 @@
 // accesses are coalesced rows of kColsPerBlock columns.
 #pragma once
 
+#include <type_traits>
+
 #include "cdns_common.cuh"
 
 namespace cdns {
@@ -218,6 +220,17 @@ template <int E> __device__ __forceinline__ int tile_slot(int y, int l) {
 inline int lane_elems(const Dims &d) {
     const int e = (d.ncy + 31) / 32;
     return e <= 1 ? 1 : e <= 2 ? 2 : e <= 4 ? 4 : e <= 8 ? 8 : 0;
+}
+
+// fn(E) for the elements per lane of this column length; false if it is too long
+template <class Fn> bool with_elems(const Dims &d, Fn &&fn) {
+    switch (lane_elems(d)) {
+    case 1: fn(std::integral_constant<int, 1>{}); return true;
+    case 2: fn(std::integral_constant<int, 2>{}); return true;
+    case 4: fn(std::integral_constant<int, 4>{}); return true;
+    case 8: fn(std::integral_constant<int, 8>{}); return true;
+    default: return false;   // more than 256 Chebyshev coefficients
+    }
 }
 
 }  // namespace cdns

@@ -1,15 +1,16 @@
 """Results whose rounding order is kept.
 
 dp/dx of a constant flow rate is (Q - q) / q_unit with Q - q some 4e-6 of Q, so that
-it shows each last bit of the flux q as 5e-11.  In the mixed form every value of the
-FP64 part is rounded to FP32 once a step, so that in a few steps another order of the
-FP64 operations leaves unrelated FP32 noise: 1e-6 in dp/dx, up to 7e-7 in the pressure.
-The golden values (golden/golden_rounding_order.npz, written by this file run as a
-program) are those of the library at commit 32f7165; in the mixed form the same order
-of operations gives the same bits.  By the chains of solver.cu the mixed dp/dx differs
-by 4e-7 to 3e-6 here and the pressure by 1e-11 to 2e-7, and the FP64 dp/dx by 5e-11
-to 2e-10 where its last bits differ at all; the bounds leave room for another last bit
-in a table or in the nonlinear term, not for that."""
+it shows each last bit of the flux q as 5e-11; the mean wall shear weights coefficient
+k of the profile by k^2.  In the mixed form every value of the FP64 part is rounded to
+FP32 once a step, so that in a few steps another order of the FP64 operations leaves
+unrelated FP32 noise: 1e-6 in dp/dx, up to 7e-7 in the pressure.  The golden values
+(golden/golden_rounding_order.npz, written by this file run as a program) are those of
+the library at commit 32f7165; in the mixed form the same order of operations gives the
+same bits.  By the chains of solver.cu the mixed dp/dx differs by 4e-7 to 3e-6 here and
+the pressure by 1e-11 to 2e-7, the FP64 dp/dx by 5e-11 to 2e-10 (or not at all, where
+its last bits happen to agree) and the shear by 7e-12 to 5e-11; the bounds leave room for
+another last bit in a table or in the nonlinear term, not for that."""
 import os
 import sys
 
@@ -34,6 +35,7 @@ MIXED = {
 }
 FP64 = {"fp64_32": (32, 48, 32, 48, 72, 48), "fp64_62": (62, 58, 40, 96, 88, 60), "fp64_102": (102, 28, 52, 162, 46, 81),
         "fp64_28": (28, 106, 24, 45, 160, 36), "fp64_130": (20, 150, 16, 32, 226, 24)}
+SHEAR = {"shear_50": (50, 26, 40, 75, 40, 63), "shear_32": (32, 28, 70, 49, 44, 108), "shear_24": (24, 24, 26, 36, 36, 40)}
 
 
 def field(mesh):
@@ -72,6 +74,15 @@ def advance(shape, flow, precision, steps):
     return np.array(ctx.dpdx()), ctx.get_pressure()[z - 3:z + 4, :, :4].copy()
 
 
+def mean_shear(shape):
+    """The wall shear averaged over 12 steps, the adjoint's objective."""
+    nx, ny, nz, nx2, ny2, nz2 = shape
+    mesh = cdns.Mesh(nx, ny, nz, nx // 2, ny - 2, nz // 2, nx2, ny2, nz2, 4.0 * PI, 2.0 * PI)
+    ctx = cdns.Context(mesh, cdns.Params(Re=180.0, DT=5e-5))
+    ctx.set_velocity(field(mesh))
+    return np.array(ctx.adjoint_run(12, 4, gradient=False)[0])
+
+
 def off(got, want):
     return np.linalg.norm(got - want) / np.linalg.norm(want)
 
@@ -91,18 +102,36 @@ def test_mixed(name, monkeypatch):
     assert off(p, want[name + "_p"]) <= 1e-12
 
 
+# FP64: launch shapes by rule, so that the nonlinear term rounds alike in every process
+BY_RULE = {"CDNS_TUNE": "0", "CDNS_X_STAGE": "rows4", "CDNS_Y_TRANSFORM": "matrix"}
+
+
+@pytest.fixture
+def by_rule(monkeypatch):
+    for k, v in BY_RULE.items():
+        monkeypatch.setenv(k, v)
+
+
 @pytest.mark.parametrize("name", list(FP64))
-def test_fp64_flow_rate(name):
+def test_fp64_flow_rate(name, by_rule):
     """Against 4e-12: 0.08 of one last bit of q."""
     dpdx, _ = advance(FP64[name], "rate", cdns.PRECISION_FP64, 6)
     assert off(dpdx, np.load(GOLDEN)[name + "_dpdx"]) <= 4e-12
+
+
+@pytest.mark.parametrize("name", list(SHEAR))
+def test_fp64_mean_shear(name, by_rule):
+    """Coefficient k of the profile counts k^2-fold: a last bit of the last ones is 1e-12."""
+    assert off(mean_shear(SHEAR[name]), np.load(GOLDEN)[name]) <= 4e-12
 
 
 if __name__ == "__main__":
     out = {}
     for n in MIXED:
         out[n + "_dpdx"], out[n + "_p"] = run_mixed(n, os.environ.__setitem__)
-    del os.environ["CDNS_X_STAGE"], os.environ["CDNS_Y_TRANSFORM"]
+    os.environ.update(BY_RULE)
     for n in FP64:
         out[n + "_dpdx"], _ = advance(FP64[n], "rate", cdns.PRECISION_FP64, 6)
+    for n in SHEAR:
+        out[n] = mean_shear(SHEAR[n])
     np.savez(sys.argv[1], **out)
